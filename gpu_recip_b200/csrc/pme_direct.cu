@@ -4,20 +4,20 @@
 // models of the reference's direct test: shifted Lennard-Jones (VDW_VSH,
 // CudaDirectForceKernels.cu:175-195) and Ewald real-space electrostatics (EWALD, :353-391).
 //
-// One calc_force is five launches on the handle's stream:
-//   k_direct_cell   atom -> cell (cells >= roff along x, >= roff/2 along y and z), counts;
-//   k_direct_scan   cell starts (one CTA);
-//   k_direct_fill   atoms into their cells (unordered);
-//   k_direct_order  one warp per cell: order the cell's atoms by index (so every run sums in the
-//                   same order) and gather coordinates, type, global index and exclusion window;
-//   k_direct_pairs  one warp per 32 atoms of a cell (lane = atom i) and z slice of its 3 x 5 x 5
-//                   neighbouring cells: a cheap distance/exclusion pass compacts the pairs within
-//                   roff, whose terms then run on full lanes.
+// One calc_force is a clear and five launches on the handle's stream:
+//   k_direct_cell     atom -> (y, z) column and x bin, counts (columns a fraction of roff wide);
+//   k_direct_columns  one warp per column: room for its atoms, first atom of every bin, clusters of 8
+//                     consecutive atoms;
+//   k_direct_fill     atoms into their bins (unordered);
+//   k_direct_order    order every bin's atoms by x and index (so every run sums in the same order) and
+//                     gather coordinates, type, global index and exclusion window;
+//   k_direct_pairs    one warp per cluster: candidates are the x intervals of the columns in reach; a
+//                     cheap FP32 distance pass queues them per atom, the pair terms then run on full
+//                     lanes.
 // Each pair is evaluated from both sides (no third-law scatter): each pair's force is rounded once
-// to 2^-40 and every sum after that is exact int64, so results are run-to-run identical and the
-// only FP32 error is that of the pair terms themselves.  Energies are rounded to 2^-32 per pair and summed in int64; both sides
-// give the same pair distance (dx = (x_i - x_j) - shift is antisymmetric), so the doubled sums
-// halve exactly (1-4 terms are added twice to match).
+// to 2^-40 and every sum after that is exact int64, so results are run-to-run identical.  Energies
+// are rounded to 2^-32 per pair and summed in int64; both sides give the same pair distance, so the
+// doubled sums halve exactly (1-4 terms are added twice to match).
 // Exclusions: a 128-bit window per atom over global indices g_j - g_i in [-64, 64) (bit 64: the
 // atom itself), plus an explicit list for partners beyond the window.
 #include <cuda_runtime.h>
@@ -33,29 +33,38 @@
 namespace pme {
 namespace direct {
 
-constexpr int kWarps = 8;             // warps per CTA of the pair kernel (256 threads)
-constexpr int kMaxTypes = 200;        // vdW types (packed pairs held in shared memory)
+constexpr int kWarps = 4;             // warps per CTA of the pair kernel
+constexpr int kPairCtas = 5;          // its CTAs per SM
+constexpr int kCluster = 8;           // i atoms of a warp task: 4 lanes share one atom
+constexpr int kQueue = 72;            // queued candidates per i atom (at most 32 more at a time)
+constexpr int kTasksPerWarp = 3;      // pair tasks per resident warp to aim at
+constexpr int kMaxReach = 4;          // columns within the cutoff on each side, at most
+constexpr int kMaxXBins = 1024;       // x look-up entries per column, at most
+constexpr int kSquareTypes = 64;      // vdW types up to which every CTA holds the full square table
+constexpr int kMaxTypes = 200;        // vdW types
 constexpr float kEnergyScale = 4294967296.0f;     // 2^32
 constexpr float kForceScaleF = 1099511627776.0f;  // 2^40
 constexpr float kTwoSqrtPi = 1.1283791670955126f; // 2/sqrt(pi)
-constexpr int kTabN = 4096;          // Ewald table intervals
-constexpr double kTabR0 = 1.5;       // Ewald table from r = 1.5 A (closer pairs use erfc and exp)
+constexpr int kTabOctave = 64, kTabMax = 16 * kTabOctave;   // Ewald table intervals (see ensure_ewald)
 
 struct Params {
   float box[3], inv_box[3];
   float kappa, kappa2, roff2, ro6, ro12, ro18;   // roff^-6, roff^-12, roff^-18
   float e14fac;
   int vdw, elec;
-  int nc[3];          // cells per axis
-  int lo[3], cnt[3];  // neighbour cell offsets per axis: lo .. lo + cnt - 1
-  int npair;          // vdW type pairs
-  double kappad, ro6d, ro12d, ro18d;   // FP64 copies for the main-list pair terms
+  int nc[3];          // x look-up bins per column; columns along y and z
+  int reach[2];       // column offsets -reach .. reach along y and z
+  float cut2, marg;   // widened squared cutoff of the cheap pass; slack of the candidate intervals (A)
+  int ntype;          // vdW types
+  int square;         // shared memory holds the vdW table as ntype x ntype (else the packed triangle is read)
+  int big_hi;         // high word of 1024 / roff: forces above it take the slow rounding
+  int slices;         // tasks per cluster, each with some of the column rows along z
+  double kappad, roff2d, ro6d, ro12d, ro18d;   // FP64 for the main-list pair terms
   double boxd[3];
-  // Ewald real-space table (Hermite cubic in s = r^2 on [tab_s0, roff^2], tab_n intervals):
-  // per node (E, h dE/ds, F, h dF/ds) with E = erfc(kappa r)/r and F = (r dE/dr) / r^2
+  // Ewald real space, cubics on the intervals of s = r^2 that share their leading float bits (kTabOctave
+  // per factor of two, from s = 2): F = (r dE/dr) / r^2 of E = erfc(kappa r) / r, then E itself
   const double4* tab;
-  double tab_s0, tab_invh;
-  int tab_n;
+  int tab_n;          // intervals (0: no table); s outside them uses erfc() and exp()
 };
 
 enum Acc { kAccVdw = 0, kAccElec = 1, kAccExcl = 2, kAccVir = 3, kAccN = 9 };   // vir: xx xy xz yy yz zz
@@ -90,37 +99,43 @@ __device__ __forceinline__ float pair_terms(float r2, float qq, float c6, float 
 // The same terms in FP64 from the FP32 pair geometry, for the main pair list: the atoms' net
 // forces are small differences of large pair forces (close contacts of ~1e3 kcal/mol/A), where
 // the few-ulp error of an FP32 evaluation shows.
-__device__ __forceinline__ double pair_terms_f64(double r2, double qq, double c6, double c12, const Params& p,
-                                                 bool vdw, double& u_vdw, double& u_elec) {
-  const double rinv = rsqrt(r2);
-  const double r = r2 * rinv;
-  const double rinv2 = rinv * rinv;
-  double fr = 0.0;
-  u_vdw = 0.0;
-  if (vdw) {
-    const double rinv6 = rinv2 * rinv2 * rinv2, rinv12 = rinv6 * rinv6, r6 = r2 * r2 * r2;
-    fr = c6 * (rinv6 - r6 * p.ro12d) - c12 * (rinv12 + r6 * p.ro18d);
+
+// 1 / x by one third-order Newton (Halley-type) step y (1 + e + e^2), e = 1 - x y, from the
+// hardware's approximation (relative error below 2^-19, so below 2^-52 after the step).
+__device__ __forceinline__ double reciprocal(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = __fma_rn(-x, y, 1.0);
+  return __fma_rn(y, __fma_rn(e, e, e), y);
+}
+
+__device__ __forceinline__ double cubic(const double2* c, double t) {
+  const double2 lo = c[0], hi = c[1];
+  return __fma_rn(__fma_rn(__fma_rn(hi.y, t, hi.x), t, lo.y), t, lo.x);
+}
+
+// Shifted Lennard-Jones: (r dU/dr) and U from s = r^2 and 1 / s.
+template <bool EV>
+__device__ __forceinline__ double vdw_terms_f64(double s, double sinv, float2 cc, const Params& p, double& u_vdw) {
+  const double c6 = cc.x, c12 = cc.y;
+  const double rinv6 = sinv * sinv * sinv, r6 = s * s * s, rinv12 = rinv6 * rinv6;
+  if (EV)
     u_vdw = c12 * (1.0 / 12.0) * (rinv12 + 2.0 * r6 * p.ro18d - 3.0 * p.ro12d) -
             c6 * (1.0 / 6.0) * (rinv6 + r6 * p.ro12d - 2.0 * p.ro6d);
-  }
+  return c6 * (rinv6 - r6 * p.ro12d) - c12 * (rinv12 + r6 * p.ro18d);
+}
+
+// All terms without the Ewald table: (r dU/dr) / r^2.
+__device__ __forceinline__ double pair_terms_f64(double s, double qq, float2 cc, const Params& p, double& u_vdw,
+                                              double& u_elec) {
+  const double rinv = rsqrt(s), r = s * rinv, sinv = rinv * rinv;
+  double fr = vdw_terms_f64<true>(s, sinv, cc, p, u_vdw);
   u_elec = 0.0;
-  if (p.elec == PME_ELEC_NONE) return fr * rinv2;
-  if (p.tab != nullptr && r2 >= p.tab_s0) {
-    const double u = (r2 - p.tab_s0) * p.tab_invh;
-    const int i = min((int)u, p.tab_n - 1);
-    const double t = u - (double)i;
-    const double2* q = reinterpret_cast<const double2*>(p.tab + i);
-    const double2 a0 = __ldg(q), a1 = __ldg(q + 1), b0 = __ldg(q + 2), b1 = __ldg(q + 3);
-    const double t2 = t * t;
-    const double h01 = t2 * (3.0 - 2.0 * t), h00 = 1.0 - h01;
-    const double h10 = t * (1.0 - t) * (1.0 - t), h11 = t2 * (t - 1.0);
-    u_elec = qq * (h00 * a0.x + h10 * a0.y + h01 * b0.x + h11 * b0.y);
-    return fr * rinv2 + qq * (h00 * a1.x + h10 * a1.y + h01 * b1.x + h11 * b1.y);
+  if (p.elec != PME_ELEC_NONE) {
+    u_elec = qq * erfc(p.kappad * r) * rinv;
+    fr += -qq * 1.1283791670955126 * p.kappad * exp(-p.kappad * p.kappad * s) - u_elec;
   }
-  const double e = qq * erfc(p.kappad * r) * rinv;
-  u_elec = e;
-  fr += -qq * 1.1283791670955126 * p.kappad * exp(-p.kappad * p.kappad * r2) - e;
-  return fr * rinv2;
+  return fr * sinv;
 }
 
 __device__ __forceinline__ float2 vdw_c6c12(const float2* tab, int ta, int tb) {
@@ -138,8 +153,8 @@ __device__ __forceinline__ long long warp_sum_ll(long long v) {
 // Binning
 // ---------------------------------------------------------------------------------------------
 // Coordinate wrapped into the box: x - L floor(x / L), which FP32 rounding can leave a hair below
-// 0 or equal to L; non-finite inputs become 0.  The cell comes from this same value, so an atom's
-// cell and its stored position always agree (the cells are wider than their reach by a margin).
+// 0 or equal to L; non-finite inputs become 0.  The column and x bin come from this same value, so
+// they and an atom's stored position always agree (the candidate intervals have that slack).
 __device__ __forceinline__ float wrap_coord(float x, float box, float inv_box) {
   const float w = x - box * floorf(x * inv_box);
   return (w >= -box && w <= 2.0f * box) ? w : 0.0f;
@@ -149,7 +164,7 @@ __device__ __forceinline__ int cell_of_wrapped(float w, float inv_box, int n) {
   return max(0, min((int)(w * inv_box * (float)n), n - 1));
 }
 
-__global__ void k_direct_cell(const float4* __restrict__ xyzq, int n, const Params p, int* __restrict__ cell_of,
+__global__ void k_direct_cell(const float4* __restrict__ xyzq, int n, const Params p, int2* __restrict__ cell_of,
                               int* __restrict__ count) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -157,81 +172,81 @@ __global__ void k_direct_cell(const float4* __restrict__ xyzq, int n, const Para
   const int cx = cell_of_wrapped(wrap_coord(a.x, p.box[0], p.inv_box[0]), p.inv_box[0], p.nc[0]);
   const int cy = cell_of_wrapped(wrap_coord(a.y, p.box[1], p.inv_box[1]), p.inv_box[1], p.nc[1]);
   const int cz = cell_of_wrapped(wrap_coord(a.z, p.box[2], p.inv_box[2]), p.inv_box[2], p.nc[2]);
-  const int c = (cz * p.nc[1] + cy) * p.nc[0] + cx;
-  cell_of[i] = c;
-  atomicAdd(&count[c], 1);
+  const int c = (cz * p.nc[1] + cy) * (p.nc[0] + 1) + cx;
+  cell_of[i] = make_int2(c, atomicAdd(&count[c], 1));
 }
 
-// Exclusive scans of count[0..ncell) into start[0..ncell] (atoms) and of ceil(count / 32) into
-// chunk[0..ncell] (32-atom chunks, chunk[ncell] the total); one CTA of 1024 threads, each owning a
-// contiguous run of cells.
-__global__ void __launch_bounds__(1024) k_direct_scan(const int* __restrict__ count, int ncell, int* __restrict__ start,
-                                                      int* __restrict__ chunk) {
-  __shared__ int part[1024], partc[1024];
-  const int t = threadIdx.x;
-  const int per = (ncell + 1023) / 1024;
-  const int b = min(t * per, ncell), e = min(b + per, ncell);
-  int s = 0, sc = 0;
-  for (int c = b; c < e; c++) {
-    s += count[c];
-    sc += (count[c] + 31) >> 5;
+// One warp per column: reserves room for the column's atoms and clusters (columns come in any order:
+// no result depends on where they lie), writes xstart[cell] = first atom of every x bin (entry nbx of
+// a column: its end) and the column's clusters (first atom, column).
+__global__ void k_direct_columns(const Params p, const int* __restrict__ count, int ncol, int* __restrict__ totals,
+                                 int* __restrict__ xstart, int2* __restrict__ clusters) {
+  const int lane = threadIdx.x & 31, nbx = p.nc[0];
+  const int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (col >= ncol) return;
+  const int* cnt = count + (size_t)col * (nbx + 1);
+  int n = 0;
+  for (int b = lane; b < nbx; b += 32) n += cnt[b];
+  n = __reduce_add_sync(0xffffffffu, n);
+  const int nc = (n + kCluster - 1) / kCluster;
+  int first = 0, clus = 0;
+  if (lane == 0 && n > 0) {
+    first = atomicAdd(&totals[0], n);
+    clus = atomicAdd(&totals[1], nc);
   }
-  part[t] = s;
-  partc[t] = sc;
-  __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {   // inclusive Hillis-Steele scans of the run sums
-    const int v = t >= off ? part[t - off] : 0;
-    const int vc = t >= off ? partc[t - off] : 0;
-    __syncthreads();
-    part[t] += v;
-    partc[t] += vc;
-    __syncthreads();
-  }
-  int run = part[t] - s, runc = partc[t] - sc;
-  for (int c = b; c < e; c++) {
-    start[c] = run;
-    chunk[c] = runc;
-    run += count[c];
-    runc += (count[c] + 31) >> 5;
-  }
-  if (t == 1023) {
-    start[ncell] = part[1023];
-    chunk[ncell] = partc[1023];
+  first = __shfl_sync(0xffffffffu, first, 0);
+  clus = __shfl_sync(0xffffffffu, clus, 0);
+  for (int k = lane; k < nc; k += 32) clusters[clus + k] = make_int2(first + k * kCluster, col);
+  int run = first;
+  for (int b0 = 0; b0 <= nbx; b0 += 32) {
+    const int b = b0 + lane, v = b < nbx ? cnt[b] : 0;
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (b <= nbx) xstart[(size_t)col * (nbx + 1) + b] = run + incl - v;
+    run += __shfl_sync(0xffffffffu, incl, 31);
   }
 }
 
-__global__ void k_direct_fill(const int* __restrict__ cell_of, int n, const int* __restrict__ start,
-                              int* __restrict__ fill, int* __restrict__ tmp) {
+// Order of an atom in its bin: by wrapped x, then by index (as one 64-bit integer).
+__device__ __forceinline__ unsigned long long order_key(float x, int atom) {
+  const unsigned int b = (unsigned int)__float_as_int(x);
+  return (unsigned long long)(b ^ ((b >> 31) ? 0xffffffffu : 0x80000000u)) << 32 | (unsigned int)atom;
+}
+
+__global__ void k_direct_fill(const int2* __restrict__ cell_of, int n, const Params p, const float4* __restrict__ xyzq,
+                              const int* __restrict__ xstart, unsigned long long* __restrict__ keys) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int c = cell_of[i];
-  tmp[start[c] + atomicAdd(&fill[c], 1)] = i;
+  const int2 c = cell_of[i];
+  keys[xstart[c.x] + c.y] = order_key(wrap_coord(xyzq[i].x, p.box[0], p.inv_box[0]), i);
 }
 
-// One warp per cell: rank each of the cell's atoms by index and gather its data to that slot.
-__global__ void k_direct_order(const int* __restrict__ start, int ncell, const int* __restrict__ tmp,
+// One thread per filled slot: rank its atom among the few of its bin and gather its data there.
+__global__ void k_direct_order(const Params p, int n, const unsigned long long* __restrict__ keys,
+                               const int2* __restrict__ cell_of, const int* __restrict__ xstart,
                                const float4* __restrict__ xyzq, const int* __restrict__ vdwtype,
                                const int* __restrict__ glob, const ulonglong2* __restrict__ win,
-                               const int* __restrict__ far_ptr, float box_x, float box_y, float box_z, float inv_x,
-                               float inv_y, float inv_z, float4* __restrict__ pos, int4* __restrict__ info,
+                               const int* __restrict__ far_ptr, float4* __restrict__ pos, int4* __restrict__ info,
                                ulonglong2* __restrict__ mask) {
-  const int lane = threadIdx.x & 31;
-  for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < ncell; c += (gridDim.x * blockDim.x) >> 5) {
-    const int s = start[c], e = start[c + 1];
-    for (int k = s + lane; k < e; k += 32) {
-      const int a = tmp[k];
-      int rank = 0;
-      for (int m = s; m < e; m++) rank += tmp[m] < a ? 1 : 0;
-      const int d = s + rank;
-      float4 q = xyzq[a];   // wrapped: neighbour cells then need only their periodic shift
-      q.x = wrap_coord(q.x, box_x, inv_x);
-      q.y = wrap_coord(q.y, box_y, inv_y);
-      q.z = wrap_coord(q.z, box_z, inv_z);
-      pos[d] = q;
-      info[d] = make_int4(vdwtype[a], glob[a], a, far_ptr[a + 1] > far_ptr[a] ? 1 : 0);
-      mask[d] = win[a];
-    }
-  }
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const unsigned long long key = keys[k];
+  const int a = (int)(unsigned int)key;
+  const int cell = cell_of[a].x;
+  const int s = xstart[cell], e = xstart[cell + 1];
+  int d = s;
+  for (int m = s; m < e; m++) d += keys[m] < key ? 1 : 0;
+  float4 q = xyzq[a];
+  q.x = wrap_coord(q.x, p.box[0], p.inv_box[0]);
+  q.y = wrap_coord(q.y, p.box[1], p.inv_box[1]);
+  q.z = wrap_coord(q.z, p.box[2], p.inv_box[2]);
+  pos[d] = q;
+  info[d] = make_int4(vdwtype[a], glob[a], a, far_ptr[a + 1] > far_ptr[a] ? 1 : 0);
+  mask[d] = win[a];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -244,219 +259,323 @@ __device__ __forceinline__ bool far_excluded(const int* __restrict__ far_ptr, co
   return false;
 }
 
-// One warp per (cell, 32-atom chunk of it, z slice of its neighbour cells): lane = atom i.  For
-// each batch of 32 j atoms staged in shared memory, a cheap pass tests the 32 x 32 pairs (distance
-// with the neighbour cell's periodic shift, or the minimum image when an axis has too few cells,
-// then the exclusion window) and compacts the hits into a per-warp list; the pair terms then run
-// in FP64 (from the FP32 positions, exactly) on full lanes, 32 hits at a time (the list is ordered
-// by i, so a segmented warp scan folds each i's run into one add to its shared-memory
-// accumulator).  Every pair force is rounded once to 2^-40 and summed in
-// int64 from there on (exact: no accumulation error, and no dependence on the order of the adds
-// or of the slices).  FP64 because an atom's net force is a small difference of large pair forces,
-// where the few-ulp error of FP32 pair terms reaches ~1e-5 kcal/mol/A.
-template <bool MINIMG>
-__global__ void __launch_bounds__(kWarps * 32, 3) k_direct_pairs(
-    const Params p, const int* __restrict__ start, const int* __restrict__ chunkp, const float4* __restrict__ pos,
-    const int4* __restrict__ info,
+// d - n L for the image number n = field - 1 (field in 0..2), n made a double by placing the field in
+// the low bits of 1.5 * 2^52.
+__device__ __forceinline__ double shift_image(double d, int field, double box) {
+  const double n = __dadd_rn(__hiloint2double(0x43380000, field), -6755399441055745.0);
+  return __fma_rn(-n, box, d);
+}
+
+// Two FP32 values in one 64-bit register and packed arithmetic on them (sm_100).
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  return (unsigned long long)(unsigned int)__float_as_int(b) << 32 | (unsigned int)__float_as_int(a);
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// Predicated 8-byte shared-memory store (an if around it costs three branch instructions).
+__device__ __forceinline__ void store_if_less(float a, float b, unsigned int addr, int x, int y) {
+  asm volatile("{\n .reg .pred p;\n setp.lt.f32 p, %0, %1;\n @p st.shared.v2.b32 [%2], {%3, %4};\n}" ::"f"(a), "f"(b),
+               "r"(addr), "r"(x), "r"(y)
+               : "memory");
+}
+
+// One warp per cluster of 8 atoms consecutive along x in a column (a compact block at liquid
+// density) and slice of its column rows.  Each column in reach contributes the x interval that the
+// cluster's bounding box can reach at that column's distance, once per periodic image.  The cheap
+// pass takes the intervals' atoms in blocks of 32 (lane = candidate), tests each against the 8 atoms
+// in FP32 with a slightly widened cutoff and queues the hits per atom in shared memory; when a queue
+// fills (or at the end), lanes 4 i .. 4 i + 3 take atom i's hits in whole rounds and run the pair
+// terms in FP64 from the exact FP32 geometry: cutoff, exclusions, forces rounded once to 2^-40 and
+// summed in int64 in registers (exact: no accumulation error and no dependence on the order).  FP64
+// because an atom's net force is a small difference of large pair forces, where the few-ulp error of
+// FP32 pair terms reaches ~1e-5 kcal/mol/A.
+// STD: vdW (square table) and Ewald (table) both on, the flags known at compile time.
+template <bool EV, bool STD>
+__global__ void __launch_bounds__(kWarps * 32, kPairCtas) k_direct_pairs(
+    const __grid_constant__ Params p, const int* __restrict__ nclus, const int2* __restrict__ clusters,
+    const int* __restrict__ xstart, const float4* __restrict__ pos, const int4* __restrict__ info,
     const ulonglong2* __restrict__ mask, const int* __restrict__ far_ptr, const int* __restrict__ far_idx,
     const float2* __restrict__ vdwp, int calc_energy, int calc_virial, int stride, long long* __restrict__ force,
     long long* __restrict__ acc, int* __restrict__ next_task) {
-  extern __shared__ float2 sh_vdw[];
-  __shared__ float4 sh_jpos[kWarps][32];
-  __shared__ int2 sh_jtg[kWarps][32];
-  __shared__ float4 sh_ipos[kWarps][32];
-  __shared__ int sh_itype[kWarps][32];
-  __shared__ long long sh_f[kWarps][3][32];   // force sums at 2^40 (exact)
-  __shared__ unsigned short sh_items[kWarps][1024];
-  for (int k = threadIdx.x; k < p.npair; k += blockDim.x) sh_vdw[k] = vdwp[k];
+  extern __shared__ double2 sh_dyn[];   // Ewald cubics (with EV: F and E of an interval together), then vdW table
+  constexpr int kEntry = EV ? 4 : 2;    // double2 per interval
+  float2* const sh_vdw = reinterpret_cast<float2*>(sh_dyn + kEntry * p.tab_n);
+  for (int k = threadIdx.x; k < kEntry * p.tab_n; k += blockDim.x)
+    sh_dyn[k] = __ldg(reinterpret_cast<const double2*>(p.tab) + (EV ? k : (k >> 1) * 4 + (k & 1)));
+  __shared__ int2 sh_queue[kWarps][kCluster][kQueue + 1];   // j and its image (2 bits per axis)
+  __shared__ ulonglong2 sh_xy[kWarps][kCluster / 2];        // the cluster's coordinates, atoms in pairs
+  __shared__ unsigned long long sh_z[kWarps][kCluster / 2];
+  if (p.square)
+    for (int k = threadIdx.x; k < p.ntype * p.ntype; k += blockDim.x) sh_vdw[k] = vdw_c6c12(vdwp, k / p.ntype, k % p.ntype);
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ncell = p.nc[0] * p.nc[1] * p.nc[2];
-  const int nslice = p.cnt[2];
+  const unsigned kFull = 0xffffffffu;
+  const double kMagic = 6755399441055744.0;   // 1.5 * 2^52: the low bits of v + kMagic hold rint(v)
+  const int kNoImage = 1 | 1 << 2 | 1 << 4;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & 3;
+  const unsigned below = (1u << lane) - 1u;
+  const unsigned int queues = (unsigned int)__cvta_generic_to_shared(&sh_queue[warp][0][0]);
   const bool vdw_on = p.vdw != PME_VDW_NONE;
+  const int ncy = p.nc[1], ncz = p.nc[2], nbx = p.nc[0];
+  const int spany = 2 * p.reach[0] + 1, spanz = 2 * p.reach[1] + 1;
+  const float wy = p.box[1] / (float)ncy, wz = p.box[2] / (float)ncz;
+  const int ntask = *nclus * p.slices;
   long long ev = 0, ee = 0;
   long long wv[6] = {0, 0, 0, 0, 0, 0};   // virial at 2^32: each task's FP64 partials folded in (exact)
-  const int nchunk = chunkp[ncell];
-  const int ntask = nchunk * nslice;
-  // tasks differ in cost (cell populations): warps take them one at a time from a counter
+  // tasks differ in cost: warps take them one at a time from a counter
   for (;;) {
     int task = 0;
     if (lane == 0) task = atomicAdd(next_task, 1);
-    task = __shfl_sync(0xffffffffu, task, 0);
+    task = __shfl_sync(kFull, task, 0);
     if (task >= ntask) break;
-    const int sl = task % nslice;
-    const int g = task / nslice;
-    int clo = 0, chi = ncell - 1;   // the cell holding chunk g: last c with chunkp[c] <= g
-    while (clo < chi) {
-      const int mid = (clo + chi + 1) >> 1;
-      if (chunkp[mid] <= g) clo = mid; else chi = mid - 1;
+    const int slice = task % p.slices;
+    const int2 cl = clusters[task / p.slices];
+    const int cy = cl.y % ncy, cz = cl.y / ncy;
+    const int i = cl.x + (lane >> 2);
+    const bool act = i < xstart[(size_t)cl.y * (nbx + 1) + nbx];
+    const float nan = __int_as_float(0x7fffffff);
+    const float4 pi = act ? pos[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int4 ii = act ? info[i] : make_int4(0, 0, 0, 0);
+    const ulonglong2 mi = act ? mask[i] : make_ulonglong2(0ull, 0ull);
+    // idle lanes: NaN coordinates, which no candidate's distance passes
+    float lo[3] = {act ? pi.x : nan, act ? pi.y : nan, act ? pi.z : nan}, hi[3] = {lo[0], lo[1], lo[2]};
+    __syncwarp();
+    if (sub == 0) {
+      const int h = (lane >> 2) & 1;
+      float* xy = reinterpret_cast<float*>(&sh_xy[warp][lane >> 3]);
+      xy[h] = lo[0];
+      xy[2 + h] = lo[1];
+      reinterpret_cast<float*>(&sh_z[warp][lane >> 3])[h] = lo[2];
     }
-    const int c = clo;
-    const int ce = start[c + 1];
-    const int cx = c % p.nc[0], cy = (c / p.nc[0]) % p.nc[1], cz = c / (p.nc[0] * p.nc[1]);
+    // bounding box of the cluster's atoms (fminf / fmaxf pass the NaN of idle lanes over)
+#pragma unroll
+    for (int d = 4; d < 32; d <<= 1)
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        lo[c] = fminf(lo[c], __shfl_xor_sync(kFull, lo[c], d));
+        hi[c] = fmaxf(hi[c], __shfl_xor_sync(kFull, hi[c], d));
+      }
+    __syncwarp();
+    long long ax = 0, ay = 0, az = 0;   // force sums at 2^40, each term plus the bits of kMagic
+    int terms = 0;                      // terms added
+    int cnt[kCluster];                  // queued hits per atom (the same on every lane)
+#pragma unroll
+    for (int q = 0; q < kCluster; q++) cnt[q] = 0;
     double w0 = 0.0, w1 = 0.0, w2 = 0.0, w3 = 0.0, w4 = 0.0, w5 = 0.0;   // this task's, in a fixed order
-    {
-      const int chunk = start[c] + (g - chunkp[c]) * 32;
-      const int i = chunk + lane;
-      const bool act = i < ce;
-      const float4 pi = act ? pos[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      const int4 ii = act ? info[i] : make_int4(0, 0, 0, 0);
-      const ulonglong2 mi = act ? mask[i] : make_ulonglong2(0ull, 0ull);
-      sh_ipos[warp][lane] = pi;
-      sh_itype[warp][lane] = ii.x;
-      sh_f[warp][0][lane] = 0;
-      sh_f[warp][1][lane] = 0;
-      sh_f[warp][2][lane] = 0;
-      // this task's z slice of the neighbour cells, with its periodic shift
-      int z = MINIMG && p.cnt[2] == p.nc[2] ? sl : cz + p.lo[2] + sl;
-      float shz = 0.0f;
-      if (!MINIMG) {
-        if (z < 0) { z += p.nc[2]; shz = -p.box[2]; } else if (z >= p.nc[2]) { z -= p.nc[2]; shz = p.box[2]; }
-      } else if (p.cnt[2] != p.nc[2]) {
-        z = (z + p.nc[2]) % p.nc[2];
-      }
-      __syncwarp();
-      for (int oy = 0; oy < p.cnt[1]; oy++) {
-        int y = MINIMG && p.cnt[1] == p.nc[1] ? oy : cy + p.lo[1] + oy;
-        float shy = 0.0f;
-        if (!MINIMG) {
-          if (y < 0) { y += p.nc[1]; shy = -p.box[1]; } else if (y >= p.nc[1]) { y -= p.nc[1]; shy = p.box[1]; }
-        } else if (p.cnt[1] != p.nc[1]) {
-          y = (y + p.nc[1]) % p.nc[1];
+    // this slice's columns, in groups of 32 (lane = column), once per x image
+    const int kend = spany * (spanz * (slice + 1) / p.slices);
+    int kcol = spany * (spanz * slice / p.slices) - 32, img = 1;
+    int col_js = 0, col_excl = 0, col_image = 0;   // this lane's column: first atom, offset in the group
+    int at = 0, total = 0;                         // candidates of the group: done, all
+    for (;;) {
+      while (at >= total && kcol < kend) {
+        // the next group of columns or x image (images -1 and +1 only where that side of the box is near)
+        if (++img > 1) {
+          img = -1;
+          kcol += 32;
+          if (kcol >= kend) break;
         }
-        for (int ox = 0; ox < p.cnt[0]; ox++) {
-          int x = MINIMG && p.cnt[0] == p.nc[0] ? ox : cx + p.lo[0] + ox;
-          float shx = 0.0f;
-          if (!MINIMG) {
-            if (x < 0) { x += p.nc[0]; shx = -p.box[0]; } else if (x >= p.nc[0]) { x -= p.nc[0]; shx = p.box[0]; }
-          } else if (p.cnt[0] != p.nc[0]) {
-            x = (x + p.nc[0]) % p.nc[0];
-          }
-          const int cn = (z * p.nc[1] + y) * p.nc[0] + x;
-          const int js = start[cn], je = start[cn + 1];
-          for (int b = js; b < je; b += 32) {
-            if (b + lane < je) {
-              sh_jpos[warp][lane] = pos[b + lane];
-              const int4 jt = info[b + lane];
-              sh_jtg[warp][lane] = make_int2(jt.x, jt.y);
-            }
-            __syncwarp();
-            const int nb = min(32, je - b);
-            // cheap pass: which of the batch's j are partners of this lane's i
-            unsigned hits = 0u;
-            if (act) {
-              for (int t = 0; t < nb; t++) {
-                const float4 pj = sh_jpos[warp][t];
-                float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-                if (MINIMG) {
-                  dx -= p.box[0] * rintf(dx * p.inv_box[0]);
-                  dy -= p.box[1] * rintf(dy * p.inv_box[1]);
-                  dz -= p.box[2] * rintf(dz * p.inv_box[2]);
-                } else {
-                  dx -= shx; dy -= shy; dz -= shz;
-                }
-                const float r2 = dx * dx + dy * dy + dz * dz;
-                if (r2 < p.roff2) {
-                  const unsigned k = (unsigned)(sh_jtg[warp][t].y - ii.y + 64);
-                  bool excl;
-                  if (k < 128u) {
-                    const unsigned long long wb = k < 64u ? mi.x : mi.y;
-                    excl = ((wb >> (k & 63u)) & 1ull) != 0ull;
-                  } else {
-                    excl = ii.w != 0 && far_excluded(far_ptr, far_idx, ii.z, sh_jtg[warp][t].y);
-                  }
-                  if (!excl) hits |= 1u << t;
-                }
-              }
-            }
-            // compact the hits, ordered by lane (i) then j
-            const int cnt = __popc(hits);
-            int off = cnt;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-              const int v = __shfl_up_sync(0xffffffffu, off, d);
-              if (lane >= d) off += v;
-            }
-            const int total = __shfl_sync(0xffffffffu, off, 31);
-            off -= cnt;
-            for (unsigned m = hits; m; m &= m - 1u) sh_items[warp][off++] = (unsigned short)((lane << 5) | (__ffs(m) - 1));
-            __syncwarp();
-            // pair terms on full lanes
-            for (int base = 0; base < total; base += 32) {
-              const bool valid = base + lane < total;
-              const int item = valid ? sh_items[warp][base + lane] : 0;
-              const int il = valid ? item >> 5 : 32 + lane;   // invalid lanes get keys of their own
-              long long gx = 0, gy = 0, gz = 0;
-              if (valid) {
-                const int t = item & 31;
-                const float4 a = sh_ipos[warp][il];
-                const float4 pj = sh_jpos[warp][t];
-                // the pair vector in FP64 from the FP32 positions (exact), image by the FP64 box
-                double ddx = (double)a.x - (double)pj.x, ddy = (double)a.y - (double)pj.y,
-                       ddz = (double)a.z - (double)pj.z;
-                if (MINIMG) {
-                  ddx -= p.boxd[0] * rint(ddx / p.boxd[0]);
-                  ddy -= p.boxd[1] * rint(ddy / p.boxd[1]);
-                  ddz -= p.boxd[2] * rint(ddz / p.boxd[2]);
-                } else {
-                  ddx -= shx == 0.0f ? 0.0 : (shx > 0.0f ? p.boxd[0] : -p.boxd[0]);
-                  ddy -= shy == 0.0f ? 0.0 : (shy > 0.0f ? p.boxd[1] : -p.boxd[1]);
-                  ddz -= shz == 0.0f ? 0.0 : (shz > 0.0f ? p.boxd[2] : -p.boxd[2]);
-                }
-                const double r2 = ddx * ddx + ddy * ddy + ddz * ddz;
-                float2 cc = make_float2(0.0f, 0.0f);
-                if (vdw_on) cc = vdw_c6c12(sh_vdw, sh_itype[warp][il], sh_jtg[warp][t].x);
-                double u_vdw, u_elec;
-                const double g = pair_terms_f64(r2, kCcelec * (double)a.w * (double)pj.w, cc.x, cc.y, p, vdw_on,
-                                                u_vdw, u_elec);
-                const double fxd = g * ddx, fyd = g * ddy, fzd = g * ddz;
-                gx = __double2ll_rn(fxd * 1099511627776.0);
-                gy = __double2ll_rn(fyd * 1099511627776.0);
-                gz = __double2ll_rn(fzd * 1099511627776.0);
-                if (calc_energy) {
-                  ev += __double2ll_rn(u_vdw * 4294967296.0);
-                  ee += __double2ll_rn(u_elec * 4294967296.0);
-                }
-                if (calc_virial) {
-                  w0 -= fxd * ddx; w1 -= fxd * ddy; w2 -= fxd * ddz;
-                  w3 -= fyd * ddy; w4 -= fyd * ddz; w5 -= fzd * ddz;
-                }
-              }
-              // segmented inclusive scan over runs of equal il (int64: exact), then one add per run
-#pragma unroll
-              for (int d = 1; d < 32; d <<= 1) {
-                const int ku = __shfl_up_sync(0xffffffffu, il, d);
-                const long long ux = __shfl_up_sync(0xffffffffu, gx, d);
-                const long long uy = __shfl_up_sync(0xffffffffu, gy, d);
-                const long long uz = __shfl_up_sync(0xffffffffu, gz, d);
-                if (lane >= d && ku == il) { gx += ux; gy += uy; gz += uz; }
-              }
-              const int kn = __shfl_down_sync(0xffffffffu, il, 1);
-              if (valid && (lane == 31 || kn != il)) {
-                sh_f[warp][0][il] += gx;
-                sh_f[warp][1][il] += gy;
-                sh_f[warp][2][il] += gz;
-              }
-              __syncwarp();
-            }
+        const float shx = (float)img * p.box[0];
+        const int k = kcol + lane;
+        int len = 0;
+        if (k < kend) {
+          const int oy = cy + k % spany - p.reach[0], oz = cz + k / spany - p.reach[1];
+          const float ylo = (float)oy * wy, zlo = (float)oz * wz;
+          const float gy = fmaxf(0.0f, fmaxf(ylo - hi[1], lo[1] - (ylo + wy)) - p.marg);
+          const float gz = fmaxf(0.0f, fmaxf(zlo - hi[2], lo[2] - (zlo + wz)) - p.marg);
+          const float rr = p.cut2 - gy * gy - gz * gz;
+          const float r = sqrtf(fmaxf(rr, 0.0f)) + p.marg;
+          const float a = lo[0] - r, b = hi[0] + r;
+          if (rr > 0.0f && (img == 0 || (img < 0 ? a < p.marg : b > p.box[0] - p.marg))) {
+            int y = oy, z = oz, iy = 1, iz = 1;
+            if (y < 0) { y += ncy; iy = 0; } else if (y >= ncy) { y -= ncy; iy = 2; }
+            if (z < 0) { z += ncz; iz = 0; } else if (z >= ncz) { z -= ncz; iz = 2; }
+            col_image = (img + 1) | iy << 2 | iz << 4;
+            const int* xs = xstart + (size_t)(z * ncy + y) * (nbx + 1);
+            col_js = xs[cell_of_wrapped(a - shx, p.inv_box[0], nbx)];
+            len = xs[cell_of_wrapped(b - shx, p.inv_box[0], nbx) + 1] - col_js;
           }
         }
+        int incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(kFull, incl, o);
+          if (lane >= o) incl += t;
+        }
+        col_excl = incl - len;
+        total = __shfl_sync(kFull, incl, 31);
+        at = 0;
       }
-      if (act) {
-        const int a = ii.z;
-        atomicAdd((unsigned long long*)&force[a], (unsigned long long)sh_f[warp][0][lane]);
-        atomicAdd((unsigned long long*)&force[a + stride], (unsigned long long)sh_f[warp][1][lane]);
-        atomicAdd((unsigned long long*)&force[a + 2 * (size_t)stride], (unsigned long long)sh_f[warp][2][lane]);
+      const bool last = at >= total;
+      if (!last) {
+        // this lane's candidate: the last column whose offset is not beyond it (empty columns share
+        // the next one's offset and are passed over)
+        const int want = at + lane;
+        int c = 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const int t = __shfl_sync(kFull, col_excl, c + o);
+          if (t <= want) c += o;
+        }
+        const int j = __shfl_sync(kFull, col_js, c) + want - __shfl_sync(kFull, col_excl, c);
+        const int jimg = __shfl_sync(kFull, col_image, c);
+        float bx = nan, by = nan, bz = nan;
+        if (want < total) {
+          const float4 pj = __ldg(&pos[j]);
+          bx = pj.x; by = pj.y; bz = pj.z;
+          if (jimg != kNoImage) {
+            bx += (float)((jimg & 3) - 1) * p.box[0];
+            by += (float)(((jimg >> 2) & 3) - 1) * p.box[1];
+            bz += (float)((jimg >> 4) - 1) * p.box[2];
+          }
+        }
+        const unsigned long long bx2 = pack2(-bx, -bx), by2 = pack2(-by, -by), bz2 = pack2(-bz, -bz);
+#pragma unroll
+        for (int h = 0; h < kCluster / 2; h++) {
+          const ulonglong2 xy = sh_xy[warp][h];
+          const unsigned long long dx = add2(xy.x, bx2), dy = add2(xy.y, by2), dz = add2(sh_z[warp][h], bz2);
+          const unsigned long long r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+#pragma unroll
+          for (int g = 0; g < 2; g++) {
+            const int q = 2 * h + g;
+            const float d2 = __int_as_float((int)(g ? r2 >> 32 : r2));
+            const unsigned m = __ballot_sync(kFull, d2 < p.cut2);
+            store_if_less(d2, p.cut2, queues + 8 * (q * (kQueue + 1) + cnt[q] + __popc(m & below)), j, jimg);
+            cnt[q] += __popc(m);
+          }
+        }
+        at += 32;
       }
+      int most = cnt[0];
+#pragma unroll
+      for (int q = 1; q < kCluster; q++) most = max(most, cnt[q]);
+      if (!last && most <= kQueue - 32) continue;
+      // pair terms, from the end of each atom's queue, 4 hits per atom and round: everything at the
+      // end, else what every atom can fill, or what the fullest queue needs to take a block more
       __syncwarp();
+      int mine = cnt[0];
+#pragma unroll
+      for (int q = 1; q < kCluster; q++) mine = (lane >> 2) == q ? cnt[q] : mine;
+      const int least = __reduce_min_sync(kFull, act ? mine : kQueue);
+      const int rounds = last ? (most + 3) >> 2 : max(least >> 2, (most - (kQueue - 32) + 3) >> 2);
+      const int2* const queue = &sh_queue[warp][lane >> 2][0];
+      const double qi = kCcelec * (double)pi.w;
+      const float2* const vrow = sh_vdw + ii.x * p.ntype;
+      for (int e = mine - 1 - sub, k = 0; k < rounds; k++, e -= 4) {
+        bool ok = e >= 0;
+        const int2 it = ok ? queue[e] : make_int2(0, kNoImage);
+        const float4 pj = __ldg(&pos[it.x]);
+        const int2 tj = __ldg(reinterpret_cast<const int2*>(&info[it.x]));   // type, global index
+        double dx = (double)pi.x - (double)pj.x, dy = (double)pi.y - (double)pj.y, dz = (double)pi.z - (double)pj.z;
+        const unsigned w = (unsigned)(tj.y - ii.y + 64);
+        if (it.y != kNoImage || w < 128u || ii.w != 0) {
+          dx = shift_image(dx, it.y & 3, p.boxd[0]);
+          dy = shift_image(dy, (it.y >> 2) & 3, p.boxd[1]);
+          dz = shift_image(dz, it.y >> 4, p.boxd[2]);
+          if (w < 128u) {   // exclusions
+            if (((w < 64u ? mi.x : mi.y) >> (w & 63u)) & 1ull) ok = false;
+          } else if (ii.w != 0 && ok) {
+            ok = !far_excluded(far_ptr, far_idx, ii.z, tj.y);
+          }
+        }
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        ok = ok && r2 < p.roff2d;
+        const double qq = qi * (double)pj.w;
+        float2 cc = make_float2(0.0f, 0.0f);
+        if (STD) cc = vrow[tj.x];
+        else if (vdw_on) cc = p.square ? vrow[tj.x] : vdw_c6c12(vdwp, ii.x, tj.x);
+        double uv = 0.0, ue = 0.0, f = 0.0;
+        bool slow = false;
+        // Ewald: the interval is the exponent and leading bits of r^2, t its offset from the middle
+        const int hi_s = __double2hiint(r2);
+        const unsigned at_s = (unsigned)(hi_s >> 14) - (0x40000000u >> 14);
+        if (STD || p.tab_n > 0) {
+          const double t = r2 - __hiloint2double((hi_s & ~0x3fff) | 0x2000, 0);
+          const double2* const c = sh_dyn + kEntry * (at_s < (unsigned)p.tab_n ? at_s : 0u);
+          f = qq * cubic(c, t);
+          if (EV) ue = qq * cubic(c + 2, t);
+        }
+        if (STD || p.elec != PME_ELEC_NONE) slow = at_s >= (unsigned)p.tab_n;
+        if (STD || vdw_on) {
+          const double sinv = reciprocal(r2);
+          f = __fma_rn(vdw_terms_f64<EV>(r2, sinv, cc, p, uv), sinv, f);
+        }
+        f = ok ? f : 0.0;
+        if (EV) {
+          uv = ok ? uv : 0.0;
+          ue = ok ? ue : 0.0;
+          slow = slow || !(fabs(uv) < 262144.0) || !(fabs(ue) < 262144.0);
+        }
+        // |f| r < 1024 unless f's high word (sign off) reaches 1024 / roff's
+        slow = ok && (slow || (__double2hiint(f) & 0x7fffffff) >= p.big_hi);
+        double fx = f * dx, fy = f * dy, fz = f * dz;
+        // rint(v 2^40) by one addition where |v| 2^40 < 2^51: the integer is the sum's low bits
+        if (!slow) {
+          ax += __double_as_longlong(__fma_rn(fx, 1099511627776.0, kMagic));
+          ay += __double_as_longlong(__fma_rn(fy, 1099511627776.0, kMagic));
+          az += __double_as_longlong(__fma_rn(fz, 1099511627776.0, kMagic));
+          terms++;
+          if (EV) {
+            const long long bits = __double_as_longlong(kMagic);
+            ev += __double_as_longlong(__fma_rn(uv, 4294967296.0, kMagic)) - bits;
+            ee += __double_as_longlong(__fma_rn(ue, 4294967296.0, kMagic)) - bits;
+          }
+        } else {   // outside the table, or a large (or non-finite) term: rounded by conversion
+          f = pair_terms_f64(r2, qq, cc, p, uv, ue);
+          fx = f * dx;
+          fy = f * dy;
+          fz = f * dz;
+          ax += __double2ll_rn(fx * 1099511627776.0);
+          ay += __double2ll_rn(fy * 1099511627776.0);
+          az += __double2ll_rn(fz * 1099511627776.0);
+          if (EV) {
+            ev += __double2ll_rn(uv * 4294967296.0);
+            ee += __double2ll_rn(ue * 4294967296.0);
+          }
+        }
+        if (EV) {
+          w0 -= fx * dx; w1 -= fx * dy; w2 -= fx * dz;
+          w3 -= fy * dy; w4 -= fy * dz; w5 -= fz * dz;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kCluster; q++) cnt[q] = max(0, cnt[q] - 4 * rounds);
+      __syncwarp();
+      if (last) break;
     }
-    if (calc_virial) {
+    // the 4 lanes of an atom join their sums; one lane per component adds it to the force array
+    const long long base = (long long)terms * __double_as_longlong(kMagic);
+    ax -= base; ay -= base; az -= base;
+#pragma unroll
+    for (int d = 1; d < 4; d <<= 1) {
+      ax += __shfl_xor_sync(kFull, ax, d);
+      ay += __shfl_xor_sync(kFull, ay, d);
+      az += __shfl_xor_sync(kFull, az, d);
+    }
+    if (act && sub < 3) {
+      const long long v = sub == 0 ? ax : (sub == 1 ? ay : az);
+      atomicAdd((unsigned long long*)&force[ii.z + (size_t)sub * stride], (unsigned long long)v);
+    }
+    if (EV) {
       wv[0] += __double2ll_rn(w0 * 4294967296.0); wv[1] += __double2ll_rn(w1 * 4294967296.0);
       wv[2] += __double2ll_rn(w2 * 4294967296.0); wv[3] += __double2ll_rn(w3 * 4294967296.0);
       wv[4] += __double2ll_rn(w4 * 4294967296.0); wv[5] += __double2ll_rn(w5 * 4294967296.0);
     }
   }
-  if (calc_energy) {
+  if (EV && calc_energy) {
     ev = warp_sum_ll(ev);
     ee = warp_sum_ll(ee);
     if (lane == 0) {
@@ -464,7 +583,7 @@ __global__ void __launch_bounds__(kWarps * 32, 3) k_direct_pairs(
       atomicAdd((unsigned long long*)&acc[kAccElec], (unsigned long long)ee);
     }
   }
-  if (calc_virial) {
+  if (EV && calc_virial) {
 #pragma unroll
     for (int q = 0; q < 6; q++) {
       const long long sv = warp_sum_ll(wv[q]);
@@ -562,17 +681,20 @@ struct pme_direct {
   int* d_far_ptr = nullptr;
   int* d_far_idx = nullptr;
   bool excl_set = false;
-  double4* d_tab = nullptr;  // Ewald real-space table for the current kappa and roff
+  double4* d_tab = nullptr;  // Ewald table for the current kappa and roff (see ensure_ewald)
+  int tab_n = 0;
   double tab_kappa = -1.0, tab_roff = -1.0;
   int4* d_list14 = nullptr;
   int n14 = 0;
   int max14 = -1;            // largest atom index in the 1-4 lists
   // per-call work space
-  int cap_atoms = 0, cap_cells = 0;
-  int* d_cell_of = nullptr;
-  int* d_tmp = nullptr;
-  int* d_count = nullptr;     // [cap_cells] counts, [cap_cells] fill counters, the pair-task counter
-  int* d_start = nullptr;     // [cap_cells + 1]
+  int cap_atoms = 0, cap_clusters = 0;
+  size_t cap_cells = 0;
+  int2* d_cell_of = nullptr;  // bin and slot of every atom
+  unsigned long long* d_keys = nullptr;
+  int* d_count = nullptr;     // [atoms placed, clusters, pair-task counter, 0], then [cap_cells] counts
+  int* d_xstart = nullptr;    // [cap_cells]: per column, its x bins and its end
+  int2* d_clusters = nullptr; // first atom and column
   float4* d_pos = nullptr;
   int4* d_info = nullptr;
   ulonglong2* d_mask = nullptr;
@@ -595,12 +717,13 @@ cudaError_t upload(T** dst, const T* src, size_t n, cudaStream_t s) {
   return e;
 }
 
-Params make_params(const pme_direct* h) {
+Params make_params(const pme_direct* h, int natom) {
   Params p;
   std::memset(&p, 0, sizeof(p));
   for (int d = 0; d < 3; d++) {
     p.box[d] = (float)h->box[d];
     p.inv_box[d] = (float)(1.0 / h->box[d]);
+    p.boxd[d] = h->box[d];
   }
   p.kappa = (float)h->kappa;
   p.kappa2 = (float)(h->kappa * h->kappa);
@@ -611,71 +734,89 @@ Params make_params(const pme_direct* h) {
   p.e14fac = (float)h->e14fac;
   p.vdw = h->vdw_model;
   p.elec = h->elec_model;
-  // cells >= roff along x (offsets -1..1) and >= roff / 2 along y and z (offsets -2..2); an axis
-  // with too few cells for distinct offsets visits each of its cells once
-  const double size[3] = {h->roff * (1.0 + 1e-5), 0.5 * h->roff * (1.0 + 1e-5), 0.5 * h->roff * (1.0 + 1e-5)};
-  const int reach[3] = {1, 2, 2};
-  for (int d = 0; d < 3; d++) {
-    p.nc[d] = std::max(1, (int)std::floor(h->box[d] / size[d]));
-    if (p.nc[d] >= 2 * reach[d] + 1) {
-      p.lo[d] = -reach[d];
-      p.cnt[d] = 2 * reach[d] + 1;
-    } else {
-      p.lo[d] = 0;
-      p.cnt[d] = p.nc[d];
-    }
-  }
-  p.npair = h->npair;
+  p.ntype = h->ntype;
+  p.square = h->ntype <= kSquareTypes ? 1 : 0;
+  const double big = 1024.0 / h->roff;
+  long long big_bits;
+  std::memcpy(&big_bits, &big, sizeof(big));
+  p.big_hi = (int)(big_bits >> 32);
   p.kappad = h->kappa;
-  for (int d = 0; d < 3; d++) p.boxd[d] = h->box[d];
-  p.tab = h->d_tab;
-  p.tab_s0 = kTabR0 * kTabR0;
-  p.tab_invh = kTabN / (h->roff * h->roff - p.tab_s0);
-  p.tab_n = kTabN;
+  p.roff2d = h->roff * h->roff;
   p.ro6d = std::pow(h->roff, -6.0);
   p.ro12d = std::pow(h->roff, -12.0);
   p.ro18d = std::pow(h->roff, -18.0);
+  const double longest = std::max(h->box[0], std::max(h->box[1], h->box[2]));
+  p.cut2 = p.roff2 * 1.00001f + (float)(1e-6 * longest * h->roff);
+  p.marg = (float)(1e-5 + 1e-6 * longest);
+  // Columns roff / reach wide (at least, by a margin) along y and z, the width nearest to the edge of
+  // a cube of kCluster atoms at the system's density, so that a cluster is about as long as wide.
+  const double edge = std::cbrt(h->box[0] * h->box[1] * h->box[2] * kCluster / std::max(natom, 1));
+  const int reach = std::max(1, std::min(kMaxReach, (int)std::lround(h->roff / edge)));
+  for (int d = 1; d < 3; d++) {
+    p.nc[d] = std::max(1, (int)std::floor(h->box[d] * reach / (h->roff * (1.0 + 1e-5))));
+    p.reach[d - 1] = reach;
+  }
+  // x bins of about 1 A (a few atoms each), 64 MB of look-up table at most
+  const double ncol = (double)p.nc[1] * p.nc[2];
+  p.nc[0] = (int)std::max(1.0, std::min({h->box[0], (double)kMaxXBins, 16.0e6 / ncol}));
+  p.tab = h->d_tab;
+  p.tab_n = h->elec_model == PME_ELEC_NONE ? 0 : h->tab_n;
   return p;
 }
 
-// Hermite table of E(s) = erfc(kappa sqrt s) / sqrt s and F(s) = (r dE/dr) / r^2 (with r dE/dr =
-// -2/sqrt(pi) kappa r exp(-kappa^2 s) - E... written per qq: the pair's r dU_elec/dr / r^2), values
-// and h-scaled s-derivatives at kTabN + 1 nodes, built in FP64 on the host.  Cubic Hermite
-// interpolation of these smooth functions at this spacing is within ~1e-9 relative.
-int ensure_table(pme_direct* h) {
+// Cubic through f at the four Chebyshev points of [mid - half, mid + half], as coefficients of 1, t,
+// t^2, t^3, t = s - mid (Newton's divided differences, expanded).
+template <class F>
+double4 chebyshev_cubic(F f, double mid, double half) {
+  double x[4], d[4];
+  for (int i = 0; i < 4; i++) {
+    x[i] = half * std::cos(kPi * (2 * i + 1) / 8.0);
+    d[i] = f(mid + x[i]);
+  }
+  for (int k = 1; k < 4; k++)
+    for (int i = 3; i >= k; i--) d[i] = (d[i] - d[i - 1]) / (x[i] - x[i - k]);
+  return make_double4(d[0] - x[0] * (d[1] - x[1] * (d[2] - x[2] * d[3])),
+                      d[1] - (x[0] + x[1]) * d[2] + (x[0] * x[1] + x[0] * x[2] + x[1] * x[2]) * d[3],
+                      d[2] - (x[0] + x[1] + x[2]) * d[3], d[3]);
+}
+
+// Table of F(s) = (r dE/dr) / s and E(s) = erfc(kappa r) / r, s = r^2, from s = 2 to roff^2 (close
+// pairs use the formulas): two cubics per interval, kTabOctave intervals per factor of two, so that
+// the interval is read off the float's leading bits.  Largest errors for r >= 1.5 A: 6e-11 of E, 3e-10
+// of F r (a cubic Hermite table of 4,096 even intervals, gathered from global memory, had 6e-11 and
+// 4e-10).  11 KB of F for roff = 9 A sit in every CTA's shared memory: two 16-byte loads and three
+// FMAs per pair, against 26 coefficients fetched and 37 FP64 operations for polynomials over the whole
+// range (192,000 atoms: 784 against 945 us).
+int ensure_ewald(pme_direct* h) {
   if (h->elec_model == PME_ELEC_NONE) return PME_OK;
-  if (h->d_tab && h->tab_kappa == h->kappa && h->tab_roff == h->roff) return PME_OK;
-  cudaFree(h->d_tab);
-  h->d_tab = nullptr;
-  const double s0 = kTabR0 * kTabR0, s1 = h->roff * h->roff;
-  if (!(s1 > s0)) return PME_OK;
-  const double k = h->kappa, c1 = 2.0 / std::sqrt(kPi) * k, hs = (s1 - s0) / kTabN;
-  std::vector<double4> t((size_t)kTabN + 1);
-  for (int i = 0; i <= kTabN; i++) {
-    const double sv = s0 + hs * i, r = std::sqrt(sv), ex = std::exp(-k * k * sv);
-    const double E = std::erfc(k * r) / r;
-    const double dEdr = (-c1 * ex * r - std::erfc(k * r)) / (r * r);
-    const double dEds = dEdr / (2.0 * r);
-    const double A = -c1 * ex - E;            // r dE/dr
-    const double F = A / sv;
-    const double dAds = c1 * k * k * ex - dEds;
-    const double dFds = (dAds * sv - A) / (sv * sv);
-    t[i] = make_double4(E, hs * dEds, F, hs * dFds);
+  if (h->tab_kappa == h->kappa && h->tab_roff == h->roff) return PME_OK;
+  h->tab_kappa = -1.0;
+  const double k = h->kappa, c1 = 2.0 / std::sqrt(kPi) * k, s1 = h->roff * h->roff;
+  std::vector<double4> t;
+  for (int i = 0; i < kTabMax; i++) {
+    const double w = std::ldexp(2.0, i / kTabOctave) / kTabOctave, a = (kTabOctave + i % kTabOctave) * w;
+    if (a > s1) break;
+    auto E = [&](double s) { const double r = std::sqrt(s); return std::erfc(k * r) / r; };
+    auto F = [&](double s) { return (-c1 * std::exp(-k * k * s) - E(s)) / s; };
+    t.push_back(chebyshev_cubic(F, a + 0.5 * w, 0.5 * w));
+    t.push_back(chebyshev_cubic(E, a + 0.5 * w, 0.5 * w));
   }
   cudaError_t e = upload(&h->d_tab, t.data(), t.size(), h->stream);
   if (e != cudaSuccess) return cuda_fail(e, "direct: Ewald table");
+  h->tab_n = (int)(t.size() / 2);
   h->tab_kappa = h->kappa;
   h->tab_roff = h->roff;
   return PME_OK;
 }
 
-int ensure_work(pme_direct* h, int n, int ncell) {
+int ensure_work(pme_direct* h, int n, int ncol, size_t ncell) {
   if (n > h->cap_atoms) {
-    cudaFree(h->d_cell_of); cudaFree(h->d_tmp); cudaFree(h->d_pos); cudaFree(h->d_info); cudaFree(h->d_mask);
-    h->d_cell_of = h->d_tmp = nullptr; h->d_pos = nullptr; h->d_info = nullptr; h->d_mask = nullptr;
+    cudaFree(h->d_cell_of); cudaFree(h->d_keys); cudaFree(h->d_pos); cudaFree(h->d_info); cudaFree(h->d_mask);
+    h->d_cell_of = nullptr; h->d_keys = nullptr; h->d_pos = nullptr; h->d_info = nullptr; h->d_mask = nullptr;
     h->cap_atoms = 0;
     const size_t m = (size_t)std::max(n, 1);
-    if (cudaMalloc(&h->d_cell_of, m * sizeof(int)) != cudaSuccess || cudaMalloc(&h->d_tmp, m * sizeof(int)) != cudaSuccess ||
+    if (cudaMalloc(&h->d_cell_of, m * sizeof(int2)) != cudaSuccess ||
+        cudaMalloc(&h->d_keys, m * sizeof(unsigned long long)) != cudaSuccess ||
         cudaMalloc(&h->d_pos, m * sizeof(float4)) != cudaSuccess || cudaMalloc(&h->d_info, m * sizeof(int4)) != cudaSuccess ||
         cudaMalloc(&h->d_mask, m * sizeof(ulonglong2)) != cudaSuccess) {
       cudaGetLastError();
@@ -684,15 +825,26 @@ int ensure_work(pme_direct* h, int n, int ncell) {
     h->cap_atoms = n;
   }
   if (ncell > h->cap_cells) {
-    cudaFree(h->d_count); cudaFree(h->d_start);
-    h->d_count = h->d_start = nullptr;
+    cudaFree(h->d_count); cudaFree(h->d_xstart);
+    h->d_count = h->d_xstart = nullptr;
     h->cap_cells = 0;
-    if (cudaMalloc(&h->d_count, (2 * (size_t)ncell + 1) * sizeof(int)) != cudaSuccess ||
-        cudaMalloc(&h->d_start, 2 * ((size_t)ncell + 1) * sizeof(int)) != cudaSuccess) {
+    if (cudaMalloc(&h->d_count, (ncell + 4) * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&h->d_xstart, ncell * sizeof(int)) != cudaSuccess) {
       cudaGetLastError();
       return fail(PME_ENOMEM, "direct: cell work space");
     }
     h->cap_cells = ncell;
+  }
+  const int nclus = n / kCluster + std::min(n, ncol) + 1;   // every column rounds up at most once
+  if (nclus > h->cap_clusters) {
+    cudaFree(h->d_clusters);
+    h->d_clusters = nullptr;
+    h->cap_clusters = 0;
+    if (cudaMalloc(&h->d_clusters, (size_t)nclus * sizeof(int2)) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(PME_ENOMEM, "direct: clusters");
+    }
+    h->cap_clusters = nclus;
   }
   return PME_OK;
 }
@@ -755,8 +907,8 @@ int pme_direct_destroy(pme_direct* h) {
   DeviceGuard dg(h->device);
   cudaStreamSynchronize(h->stream);
   for (void* p : {(void*)h->d_vdw, (void*)h->d_vdw14, (void*)h->d_vdwtype, (void*)h->d_glob, (void*)h->d_win,
-                  (void*)h->d_far_ptr, (void*)h->d_far_idx, (void*)h->d_list14, (void*)h->d_tab, (void*)h->d_cell_of, (void*)h->d_tmp,
-                  (void*)h->d_count, (void*)h->d_start, (void*)h->d_pos, (void*)h->d_info, (void*)h->d_mask,
+                  (void*)h->d_far_ptr, (void*)h->d_far_idx, (void*)h->d_list14, (void*)h->d_tab, (void*)h->d_cell_of, (void*)h->d_keys,
+                  (void*)h->d_count, (void*)h->d_xstart, (void*)h->d_clusters, (void*)h->d_pos, (void*)h->d_info, (void*)h->d_mask,
                   (void*)h->d_acc})
     if (p) cudaFree(p);
   delete h;
@@ -922,42 +1074,45 @@ int pme_direct_calc_force(pme_direct* h, const void* xyzq, int ncoord, int calc_
     h->n_types = ncoord;
     h->max_type = 0;
   }
-  if (int rc = ensure_table(h)) return rc;
-  Params p = make_params(h);
-  if (h->vdw_model == PME_VDW_NONE) p.npair = 0;
-  const int ncell = p.nc[0] * p.nc[1] * p.nc[2];
-  if (int rc = ensure_work(h, ncoord, ncell)) return rc;
+  if (int rc = ensure_ewald(h)) return rc;
+  Params p = make_params(h, ncoord);
+  if (h->vdw_model == PME_VDW_NONE) p.ntype = 0;
+  const int ncol = p.nc[1] * p.nc[2];
+  const size_t ncell = (size_t)ncol * (p.nc[0] + 1);
+  if (int rc = ensure_work(h, ncoord, ncol, ncell)) return rc;
   cudaStream_t s = h->stream;
-  cudaError_t e = cudaMemsetAsync(h->d_count, 0, (2 * (size_t)ncell + 1) * sizeof(int), s);   // + task counter
+  int* const count = h->d_count + 4;
+  cudaError_t e = cudaMemsetAsync(h->d_count, 0, (ncell + 4) * sizeof(int), s);
   if (e != cudaSuccess) return cuda_fail(e, "direct: clear counts");
   const int nb = (ncoord + 255) / 256;
-  k_direct_cell<<<nb, 256, 0, s>>>((const float4*)xyzq, ncoord, p, h->d_cell_of, h->d_count);
-  k_direct_scan<<<1, 1024, 0, s>>>(h->d_count, ncell, h->d_start, h->d_start + ncell + 1);
-  k_direct_fill<<<nb, 256, 0, s>>>(h->d_cell_of, ncoord, h->d_start, h->d_count + ncell, h->d_tmp);
+  k_direct_cell<<<nb, 256, 0, s>>>((const float4*)xyzq, ncoord, p, h->d_cell_of, count);
+  k_direct_columns<<<(ncol + 3) / 4, 128, 0, s>>>(p, count, ncol, h->d_count, h->d_xstart, h->d_clusters);
+  k_direct_fill<<<nb, 256, 0, s>>>(h->d_cell_of, ncoord, p, (const float4*)xyzq, h->d_xstart, h->d_keys);
+  k_direct_order<<<nb, 256, 0, s>>>(p, ncoord, h->d_keys, h->d_cell_of, h->d_xstart, (const float4*)xyzq, h->d_vdwtype,
+                                    h->d_glob, h->d_win, h->d_far_ptr, h->d_pos, h->d_info, h->d_mask);
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-  const int og = std::min((ncell + 7) / 8, sms * 16);
-  k_direct_order<<<og, 256, 0, s>>>(h->d_start, ncell, h->d_tmp, (const float4*)xyzq, h->d_vdwtype, h->d_glob,
-                                    h->d_win, h->d_far_ptr, p.box[0], p.box[1], p.box[2], p.inv_box[0],
-                                    p.inv_box[1], p.inv_box[2], h->d_pos, h->d_info, h->d_mask);
-  // neighbour cells by periodic shift when every axis has distinct offsets, else minimum image
-  const bool minimg = p.cnt[0] == p.nc[0] || p.cnt[1] == p.nc[1] || p.cnt[2] == p.nc[2];
-  auto kern = minimg ? k_direct_pairs<true> : k_direct_pairs<false>;
-  const size_t smem = (size_t)std::max(p.npair, 1) * sizeof(float2);
+  const bool ev = calc_energy || calc_virial;
+  const bool std_terms = h->vdw_model != PME_VDW_NONE && p.square && p.tab_n > 0;
+  auto kern = std_terms ? (ev ? k_direct_pairs<true, true> : k_direct_pairs<false, true>)
+                        : (ev ? k_direct_pairs<true, false> : k_direct_pairs<false, false>);
+  const size_t smem = (size_t)p.tab_n * (ev ? 2 : 1) * sizeof(double4) +
+                      (size_t)(p.square ? p.ntype * p.ntype : 0) * sizeof(float2);
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 48 * 1024));
   if (e != cudaSuccess) return cuda_fail(e, "direct: shared memory");
-  // chunks are counted on the device: enough CTAs for every (chunk, z slice) task of a uniform
-  // system, each warp striding over the rest
-  // one wave of resident CTAs; their warps draw the (chunk, z slice) tasks from a counter
+  // one wave of resident CTAs; their warps draw the tasks from a counter.  Few clusters: more tasks
+  // each, so that the last ones to finish are short
   int occ = 1;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kWarps * 32, smem);
   if (e != cudaSuccess) return cuda_fail(e, "direct: occupancy");
-  const long long tasks = (long long)((ncoord + 31) / 32 + ncell) * p.cnt[2];
-  const int pg = (int)std::max<long long>(1, std::min<long long>((tasks + kWarps - 1) / kWarps,
-                                                                 (long long)sms * std::max(occ, 1)));
-  kern<<<pg, kWarps * 32, smem, s>>>(p, h->d_start, h->d_start + ncell + 1, h->d_pos, h->d_info, h->d_mask,
+  const long long warps = (long long)sms * std::max(occ, 1) * kWarps;
+  const long long nclus = ncoord / kCluster + 1;
+  p.slices = (int)std::max<long long>(1, std::min<long long>((kTasksPerWarp * warps + nclus - 1) / nclus, 2 * p.reach[1] + 1));
+  const long long tasks = (long long)h->cap_clusters * p.slices;
+  const int pg = (int)std::max<long long>(1, std::min<long long>((tasks + kWarps - 1) / kWarps, warps / kWarps));
+  kern<<<pg, kWarps * 32, smem, s>>>(p, h->d_count + 1, h->d_clusters, h->d_xstart, h->d_pos, h->d_info, h->d_mask,
                                      h->d_far_ptr, h->d_far_idx, h->d_vdw, calc_energy ? 1 : 0, calc_virial ? 1 : 0,
-                                     stride, force, h->d_acc, h->d_count + 2 * ncell);
+                                     stride, force, h->d_acc, h->d_count + 2);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "direct: launch");
   return PME_OK;
@@ -978,7 +1133,7 @@ int pme_direct_calc_14_force(pme_direct* h, const void* xyzq, int calc_energy, i
     if (h->max_type >= h->ntype14) return fail(PME_EINVAL, "direct 14: a vdW type is beyond the 1-4 table");
   }
   DeviceGuard dg(h->device);
-  const Params p = make_params(h);
+  const Params p = make_params(h, 0);
   k_direct_14<<<(h->n14 + 255) / 256, 256, 0, h->stream>>>(p, h->d_list14, h->n14, (const float4*)xyzq, h->d_vdwtype,
                                                            h->d_vdw14, calc_energy ? 1 : 0, calc_virial ? 1 : 0,
                                                            stride, force, h->d_acc);

@@ -225,3 +225,54 @@ def test_direct_vdw_only(cuda, oracle):
     assert np.sqrt(((f - fo) ** 2).sum() / (fo ** 2).sum()) <= 1e-6
     assert abs(e["vdw"] - ev) <= 1e-6 * abs(ev)
     dr.close()
+
+
+@pytest.mark.parametrize("box,n,roff,ntype,kappa", [
+    ((18.0, 18.0, 18.0), 1, 9.0, 0, 0.35),          # one atom; a cutoff of half the box
+    ((18.0, 18.0, 18.0), 9, 9.0, 0, 0.35),          # partial clusters, columns visited at several images
+    ((18.0, 18.0, 18.0), 1500, 9.0, 0, 0.35),
+    ((20.0, 22.0, 19.0), 12000, 9.0, 0, 0.35),      # dense: narrow columns, queues that fill
+    ((200.0, 150.0, 180.0), 500, 9.0, 0, 0.35),     # sparse: wide columns, long clusters
+    ((18.1, 40.0, 90.0), 3000, 7.0, 0, 0.0),        # uneven box, plain Coulomb
+    ((60.0, 40.0, 45.0), 1000, 20.0, 0, 0.25),      # a long cutoff
+    ((24.0, 24.0, 24.0), 216, 9.0, 3, 0.35),        # vdW types in the square table
+    ((24.0, 24.0, 24.0), 216, 9.0, 70, 0.35),       # more types than the square table holds
+])
+def test_direct_cluster_edges_match_oracle(cuda, oracle, box, n, roff, ntype, kappa):
+    """Cluster and column edges of the pair kernel.  Forces, energies and virial are sums of FP64 terms
+    rounded once to 2^-40 and 2^-32; the parameters are exact in FP32, so 1e-8 leaves room for the
+    Ewald table (3e-10 per pair) and the rounding of sums that cancel."""
+    from gpu_recip_b200.direct import CudaPMEDirectForce, EWALD, VDW_NONE, VDW_VSH
+    rng = np.random.default_rng(n + ntype)
+    x = np.empty((n, 4), np.float32)
+    if ntype:   # in the box: wrapping a coordinate in FP32 would move it by up to its last bit (1e-6 A)
+        x[:, :3] = np.mod(_lattice()["xyzq"][:, :3], np.float32(24.0))
+    else:
+        x[:, :3] = rng.random((n, 3)) * np.array(box) * 0.999999
+    x[:, 3] = rng.integers(-8, 9, n) / 16.0
+    dr = CudaPMEDirectForce()
+    dr.setup(*box, kappa, roff, roff - 1.5, 1.0, VDW_VSH if ntype else VDW_NONE, EWALD)
+    vp, vt = np.zeros(2), np.zeros(n, np.int32)
+    if ntype:
+        vp = np.float32(rng.random(ntype * (ntype + 1))).astype(np.float64) * np.tile([1.0e2, 1.0e5], ntype * (ntype + 1) // 2)
+        vp = vp.astype(np.float32).astype(np.float64)
+        vt = rng.integers(0, ntype, n).astype(np.int32)
+        dr.set_vdwparam(vp)
+        dr.set_vdwtype(vt)
+        vp = np.stack([(6 * vp[0::2].astype(np.float32)).astype(np.float64) / 6,
+                       (12 * vp[1::2].astype(np.float32)).astype(np.float64) / 12], 1).reshape(-1)
+    xd = cuda.from_numpy(x).cuda()
+    stride = ((n + 63) // 64) * 64
+    fi, e, vir = _run(cuda, dr, xd, n, stride)
+    fo, ev, ee, vo = oracle.direct_force(x.astype(np.float64), np.array(box), kappa, roff, vp, vt,
+                                         np.zeros(n + 1, np.int32), np.zeros(0, np.int32))
+    f = fi.astype(np.float64) / FORCE_SCALE
+    assert np.sqrt(((f - fo) ** 2).sum()) <= 1e-8 * np.sqrt((fo ** 2).sum()) + 1e-9
+    assert abs(e["vdw"] - ev) <= 1e-8 * abs(ev) + 1e-6 and abs(e["elec"] - ee) <= 1e-8 * abs(ee) + 1e-6
+    assert np.abs(vir - vo).max() <= 1e-7 * np.abs(vo).max() + 1e-6
+    fi2, e2, vir2 = _run(cuda, dr, xd, n, stride)      # the forces-only kernel and the same sums again
+    fz = cuda.zeros(3 * stride, dtype=cuda.int64, device="cuda")
+    dr.calc_force(xd, n, False, False, stride, fz)
+    assert np.array_equal(fi, fi2) and e == e2 and np.array_equal(vir, vir2)
+    assert np.array_equal(fi, fz.view(3, stride)[:, :n].T.cpu().numpy())
+    dr.close()
