@@ -111,9 +111,8 @@ __host__ __device__ inline int tiles_plane(const SysDesc& d) { return d.g.hx; }
 __host__ __device__ inline int bin_tile_atoms(const SysDesc& d) { return d.bin_atoms > 0 ? d.bin_atoms : kThreads; }
 __host__ __device__ inline int tiles_bin(const SysDesc& d) { return (d.natom + bin_tile_atoms(d) - 1) / bin_tile_atoms(d); }
 __host__ __device__ inline int tiles_blocks(const SysDesc& d) { return d.nby * d.nbz; }
-// Lanes per atom of the gather (staged and fused): as few as keep the rows of one lane,
-// P^2 / lanes, at 8-9, so that a bin's atoms take few passes.
-__host__ __device__ constexpr int gather_lanes(int order) { return order <= 4 ? 2 : (order <= 6 ? 4 : 8); }
+// Lanes per atom of the gather (staged and fused): one per stencil column along x, a power of two.
+__host__ __device__ constexpr int gather_lanes(int order) { return order <= 4 ? 4 : 8; }
 constexpr int kGatherAtoms = kThreads / 8;   // staged gather tile: atoms of the smallest pass
 __host__ __device__ inline int tiles_gather(const SysDesc& d) {
   const int app = kThreads / gather_lanes(d.order);
@@ -1338,17 +1337,15 @@ __device__ __forceinline__ void finalize_system(const SysDesc& d, bool solve, bo
 }
 
 // ---------------------------------------------------------------------------------------------
-// Gather of one atom by LPA lanes (2, 4 or 8).  The P^2 stencil rows (b, c), r = b + P c, fall
-// into 8 groups r mod 8; each group's rows are summed in order of r, then the 8 group sums are
-// combined by the same pairwise tree whatever LPA is (groups g and g^4, then g^2, then g^1), the
-// pairs on one lane added locally and the others by shuffles.  Every LPA therefore gives the same
-// bits, so the staged and the fused gather agree however many lanes each gives an atom.
+// Gather of one atom by LPA = gather_lanes(P) neighbouring lanes, one per stencil column along x
+// (order 6 leaves two of 8 lanes without a column): every load of the P^2 rows reads P consecutive
+// floats of one row per atom, 4 or 8 rows per warp instruction, where lanes that took whole rows read 32
+// rows at a time (the L1 looked up about 15 lines per instruction).  A lane sums its column over y,
+// then over z; the lanes' sums are combined by a fixed shuffle tree, so the staged and the fused gather
+// give the same bits.  Bound by L1 look-ups and load latency.  Whole evaluations before and after:
+// 54,000 atoms, 90 x 75 x 80, order 8 214 and 187 us; 1,008,000 atoms, 216^3, order 6 1,247 and 1,194 us
+// (gather phase 327 and 275); 24,000 atoms, 64^3, order 6 74.6 and 71.3 us.
 // F_d = q ccelec n_d r_d sum(...) (gradient convention, CudaPMERecip.cu:1234-1242).
-template <int P>
-struct GatherSplines {
-  float thx[P], dthx[P], thy[P], dthy[P], thz[P], dthz[P];
-  int xs[P];
-};
 
 // Where a gather reads the solved real grid: the global rgrid, or (GX) a window of rows in shared
 // memory: row t = j + ry i holds grid row (y0 + j, z0 + i) wrapped, x fastest; every atom of the
@@ -1358,72 +1355,48 @@ struct RowWin {
   int y0, z0, ry;
 };
 
-// Sum of the rows r = g, g+8, g+16, ... < P^2 (group g) for the three force components.
-template <int P, bool GX = false>
-__device__ __forceinline__ float3 gather_group(const SysDesc& d, const GatherSplines<P>& sp, int g, int iy, int iz,
-                                               bool valid, const RowWin& w) {
-  const Geom& gm = d.g;
-  constexpr int RPG = (P * P + 7) / 8;
-  float f1 = 0.0f, f2 = 0.0f, f3 = 0.0f;
-#pragma unroll
-  for (int rr = 0; rr < RPG; rr++) {
-    const int r = g + 8 * rr;
-    if (valid && r < P * P) {
-      const int b = r % P, c = r / P;
-      float wy = 0.0f, dwy = 0.0f, wz = 0.0f, dwz = 0.0f;
-#pragma unroll
-      for (int q = 0; q < P; q++) {
-        if (q == b) { wy = sp.thy[q]; dwy = sp.dthy[q]; }
-        if (q == c) { wz = sp.thz[q]; dwz = sp.dthz[q]; }
-      }
-      const float* row;
-      if (GX) {
-        row = w.rows + (size_t)gm.nx * ((iy - w.y0 + b) + w.ry * (iz - w.z0 + c));
-      } else {
-        const int y = wrap_add(iy, b, gm.ny), z = wrap_add(iz, c, gm.nz);
-        row = d.rgrid + (size_t)gm.nx * (y + (size_t)gm.ny * z);
-      }
-      float s1 = 0.0f, s2 = 0.0f;
-#pragma unroll
-      for (int i = 0; i < P; i++) {
-        const float v = row[sp.xs[i]];
-        s1 = fmaf(sp.dthx[i], v, s1);
-        s2 = fmaf(sp.thx[i], v, s2);
-      }
-      f1 = fmaf(s1, wy * wz, f1);
-      f2 = fmaf(s2, dwy * wz, f2);
-      f3 = fmaf(s2, wy * dwz, f3);
-    }
-  }
-  return make_float3(f1, f2, f3);
-}
-
-__device__ __forceinline__ float3 add3(float3 a, float3 b) { return make_float3(a.x + b.x, a.y + b.y, a.z + b.z); }
-
 template <int P, int KIND, int LPA, bool GX = false>
 __device__ __forceinline__ void gather_core(const SysDesc& d, int atom, bool valid, int gl, int ix, int iy, int iz,
                                             float ux, float uy, float uz, float q,
                                             const RowWin& w = RowWin{nullptr, 0, 0, 0}) {
-  static_assert(LPA == 2 || LPA == 4 || LPA == 8, "lanes per atom");
+  static_assert(LPA == gather_lanes(P) && LPA >= P, "a lane per stencil column");
   const Geom& g = d.g;
-  GatherSplines<P> sp;
-  bspline<P>(ux, sp.thx, sp.dthx);
-  bspline<P>(uy, sp.thy, sp.dthy);
-  bspline<P>(uz, sp.thz, sp.dthz);
+  // this lane's x weight and derivative (zero for a lane beyond the stencil), all y and z weights
+  float tx = 0.0f, dx = 0.0f;
+  {
+    float th[P], dth[P];
+    bspline<P>(ux, th, dth);
 #pragma unroll
-  for (int i = 0; i < P; i++) sp.xs[i] = wrap_add(ix, i, g.nx);
-  // this lane's groups gl + LPA m, combined locally in the tree's order
-  float3 f;
-  if (LPA == 8) {
-    f = gather_group<P, GX>(d, sp, gl, iy, iz, valid, w);
-  } else if (LPA == 4) {
-    f = add3(gather_group<P, GX>(d, sp, gl, iy, iz, valid, w), gather_group<P, GX>(d, sp, gl + 4, iy, iz, valid, w));
-  } else {
-    const float3 a = add3(gather_group<P, GX>(d, sp, gl, iy, iz, valid, w),
-                          gather_group<P, GX>(d, sp, gl + 4, iy, iz, valid, w));
-    const float3 b = add3(gather_group<P, GX>(d, sp, gl + 2, iy, iz, valid, w),
-                          gather_group<P, GX>(d, sp, gl + 6, iy, iz, valid, w));
-    f = add3(a, b);
+    for (int i = 0; i < P; i++)
+      if (i == gl) { tx = th[i]; dx = dth[i]; }
+  }
+  float ty[P], dy[P], tz[P], dz[P];
+  bspline<P>(uy, ty, dy);
+  bspline<P>(uz, tz, dz);
+  float3 f = make_float3(0.0f, 0.0f, 0.0f);
+  if (valid) {
+    const int x = wrap_add(ix, gl < P ? gl : P - 1, g.nx);
+    int yo[P];
+#pragma unroll
+    for (int b = 0; b < P; b++) yo[b] = GX ? g.nx * b : g.nx * wrap_add(iy, b, g.ny);
+#pragma unroll
+    for (int c = 0; c < P; c++) {
+      const float* col = GX ? w.rows + x + g.nx * ((iy - w.y0) + w.ry * (iz - w.z0 + c))
+                            : d.rgrid + x + (size_t)(g.nx * g.ny) * wrap_add(iz, c, g.nz);
+      float s = 0.0f, t = 0.0f;
+#pragma unroll
+      for (int b = 0; b < P; b++) {
+        const float v = col[yo[b]];
+        s = fmaf(ty[b], v, s);
+        t = fmaf(dy[b], v, t);
+      }
+      f.x = fmaf(s, tz[c], f.x);
+      f.y = fmaf(t, tz[c], f.y);
+      f.z = fmaf(s, dz[c], f.z);
+    }
+    f.x *= dx;
+    f.y *= tx;
+    f.z *= tx;
   }
 #pragma unroll
   for (int off = LPA / 2; off >= 1; off >>= 1) {
