@@ -195,7 +195,6 @@ int launch_fused_single(pme_recip* h, const SysDesc& d_in) {
       h->no_cluster = true;   // this device cannot hold the cluster launch: never try again
     }
   }
-  d.gsort = gather_sorts(d, smem);
   a.nbar = fused_barriers(a.total);
   a.single = d;
   e = fused_launch(a, shape, smem, h->stream);
@@ -813,7 +812,6 @@ int pme_batch_commit(pme_batch* b) {
     smem = std::max(smem, fused_smem_bytes(b->desc[i]));
   }
   for (int p = 0; p < kPhases; p++) b->total[p] = prefix[(size_t)p * (nsys + 1) + nsys];
-  for (int i = 0; i < nsys; i++) b->desc[i].gsort = gather_sorts(b->desc[i], smem);
   cudaError_t e = cudaStreamSynchronize(b->stream);
   if (e == cudaSuccess) e = cudaMemcpy(b->d_desc, b->desc.data(), sizeof(SysDesc) * nsys, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->d_prefix, prefix.data(), prefix.size() * sizeof(int), cudaMemcpyHostToDevice);

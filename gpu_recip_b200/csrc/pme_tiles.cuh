@@ -71,8 +71,6 @@ struct SysDesc {
   int xyzq_host;             // 1: xyzq is pinned host memory, read once in index order
   int gx;                    // 1: each gather tile runs the inverse x pass of the rows it reads
                              // (fused path; no x-inverse phase)
-  int gsort;                 // 1: each gather tile (without gx) takes its atoms in order of their
-                             // stencil origin along x (a counting sort in shared memory)
   // Atom bins of the fused path: bin (by, bz) holds the atoms whose stencil origin (iy0, iz0)
   // lies in row block [by*bry, by*bry+bry) x [bz*brz, bz*brz+brz); fixed capacity bin_cap per bin,
   // surplus atoms go to an overflow list.  Counters are double-buffered by launch parity.
@@ -1513,61 +1511,7 @@ __device__ __forceinline__ RowWin gx_rows(const SysDesc& d, int y0, int z0, char
   return RowWin{rows, y0, z0, RY};
 }
 
-// Shared memory of the x-sorted order of a gather tile's atoms: 64 bytes of reduction space, a
-// histogram of nx + 1 counts, the sorted slot indices of up to bin_cap atoms.
-__host__ __device__ inline size_t gsort_smem_bytes(int nx, int bin_cap) {
-  return 64 + sizeof(int) * ((size_t)nx + 1 + (size_t)bin_cap);
-}
-
-// Whether a system's gather tiles sort their atoms by x: only without the gather's own inverse x
-// pass, where the sort's shared memory fits in what the launch takes (smem), and where bins are
-// dense (at least 128 atoms per bin on average; measured: 216^3 with ~194 atoms per bin 2.6%
-// faster per evaluation, 64^3 systems with ~94 atoms per bin 5-10% slower).  Only the throughput
-// build of the fused kernel has the sorting gather; the latency build ignores the flag.
-__host__ inline int gather_sorts(const SysDesc& d, size_t smem) {
-  const int nb = d.nby * d.nbz;
-  return (!d.gx && gsort_smem_bytes(d.g.nx, d.bin_cap) <= smem && nb > 0 && d.natom >= 128 * nb) ? 1 : 0;
-}
-
-// The slots 0..cnt-1 of a bin's records ordered by the atoms' stencil origin ix (counting sort in
-// shared memory; equal origins in any order): the atoms that one warp gathers together then read
-// the same few sectors of each grid row.  Returns the order array in shared memory.
-template <int P>
-__device__ __forceinline__ const int* gather_order_by_x(const SysDesc& d, const float* list, int cnt, char* smem_raw) {
-  constexpr int RF = rec_floats(P);
-  const int nx = d.g.nx, tid = threadIdx.x, lane = tid & 31;
-  int* hist = (int*)(smem_raw + 64);
-  int* order = hist + nx + 1;
-  for (int i = tid; i <= nx; i += kThreads) hist[i] = 0;
-  __syncthreads();
-  for (int j = tid; j < cnt; j += kThreads) atomicAdd(&hist[__float_as_int(__ldcg(list + (size_t)j * RF)) + 1], 1);
-  __syncthreads();
-  if (tid < 32) {   // exclusive starts: hist[b] = atoms with origin < b
-    const int per = (nx + 1 + 31) / 32, b0 = lane * per;
-    int s = 0;
-    for (int b = b0; b < min(b0 + per, nx + 1); b++) s += hist[b];
-    int incl = s;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    int run = incl - s;
-    for (int b = b0; b < min(b0 + per, nx + 1); b++) {
-      run += hist[b];
-      hist[b] = run;
-    }
-  }
-  __syncthreads();
-  for (int j = tid; j < cnt; j += kThreads) {
-    const int ix = __float_as_int(__ldcg(list + (size_t)j * RF));
-    order[atomicAdd(&hist[ix], 1)] = j;
-  }
-  __syncthreads();
-  return order;
-}
-
-template <int P, int KIND, int LPA, bool GX = false, bool SORT = false>
+template <int P, int KIND, int LPA, bool GX = false>
 __device__ __forceinline__ void gather_bin_tile(const SysDesc& d, int tile, int parity, char* smem_raw) {
   constexpr int RF = rec_floats(P);
   const int nbins = d.nby * d.nbz;
@@ -1578,7 +1522,6 @@ __device__ __forceinline__ void gather_bin_tile(const SysDesc& d, int tile, int 
   const int* counts = d.bin_count + parity * nbins;
   const int cnt = min(__ldcg(&counts[tile]), d.bin_cap);
   const float* list = d.bin_recs + (size_t)tile * d.bin_cap * RF;
-  const int* order = SORT ? gather_order_by_x<P>(d, list, cnt, smem_raw) : nullptr;
   constexpr int APP = kThreads / LPA;         // atoms per pass
   const int gl = tid % LPA, slot = tid / LPA;
   step_mark(d, 24);
@@ -1591,9 +1534,8 @@ __device__ __forceinline__ void gather_bin_tile(const SysDesc& d, int tile, int 
   }
   float4 h = make_float4(0.0f, 0.0f, 0.0f, 0.0f), u = h;
   if (slot < cnt) {
-    const int r = SORT ? order[slot] : slot;
-    h = __ldcg((const float4*)(list + (size_t)r * RF));
-    u = __ldcg((const float4*)(list + (size_t)r * RF + RF - 4));
+    h = __ldcg((const float4*)(list + (size_t)slot * RF));
+    u = __ldcg((const float4*)(list + (size_t)slot * RF + RF - 4));
   }
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) {
@@ -1621,17 +1563,15 @@ __device__ __forceinline__ void gather_bin_tile(const SysDesc& d, int tile, int 
     constexpr bool kPrefetch = P <= 4;
     float4 hn = make_float4(0.0f, 0.0f, 0.0f, 0.0f), un = hn;
     if (kPrefetch && j + APP < cnt) {
-      const int r = SORT ? order[j + APP] : j + APP;
-      hn = __ldcg((const float4*)(list + (size_t)r * RF));
-      un = __ldcg((const float4*)(list + (size_t)r * RF + RF - 4));
+      hn = __ldcg((const float4*)(list + (size_t)(j + APP) * RF));
+      un = __ldcg((const float4*)(list + (size_t)(j + APP) * RF + RF - 4));
     }
     if (!kPrefetch && j0 > 0) {
       h = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       u = h;
       if (valid) {
-        const int r = SORT ? order[j] : j;
-        h = __ldcg((const float4*)(list + (size_t)r * RF));
-        u = __ldcg((const float4*)(list + (size_t)r * RF + RF - 4));
+        h = __ldcg((const float4*)(list + (size_t)j * RF));
+        u = __ldcg((const float4*)(list + (size_t)j * RF + RF - 4));
       }
     }
     const int atom = __float_as_int(h.w);
@@ -1683,21 +1623,21 @@ __device__ __forceinline__ void gather_dispatch(const SysDesc& d, int tile) {
   }
 }
 
-template <int P, bool GX, bool SORT>
+template <int P, bool GX>
 __device__ __forceinline__ void gather_bin_any(const SysDesc& d, int tile, int parity, char* smem) {
   switch (d.force_kind) {
-    case kForceF32Soa: gather_bin_tile<P, kForceF32Soa, gather_lanes(P), GX, SORT>(d, tile, parity, smem); break;
-    case kForceF32x3: gather_bin_tile<P, kForceF32x3, gather_lanes(P), GX, SORT>(d, tile, parity, smem); break;
-    default: gather_bin_tile<P, kForceI64SoaAccum, gather_lanes(P), GX, SORT>(d, tile, parity, smem); break;
+    case kForceF32Soa: gather_bin_tile<P, kForceF32Soa, gather_lanes(P), GX>(d, tile, parity, smem); break;
+    case kForceF32x3: gather_bin_tile<P, kForceF32x3, gather_lanes(P), GX>(d, tile, parity, smem); break;
+    default: gather_bin_tile<P, kForceI64SoaAccum, gather_lanes(P), GX>(d, tile, parity, smem); break;
   }
 }
 
-template <bool GX, bool SORT = false>
+template <bool GX>
 __device__ __forceinline__ void gather_bin_order(const SysDesc& d, int tile, int parity, char* smem) {
   switch (d.order) {
-    case 4: gather_bin_any<4, GX, SORT>(d, tile, parity, smem); break;
-    case 6: gather_bin_any<6, GX, SORT>(d, tile, parity, smem); break;
-    default: gather_bin_any<8, GX, SORT>(d, tile, parity, smem); break;
+    case 4: gather_bin_any<4, GX>(d, tile, parity, smem); break;
+    case 6: gather_bin_any<6, GX>(d, tile, parity, smem); break;
+    default: gather_bin_any<8, GX>(d, tile, parity, smem); break;
   }
 }
 
