@@ -162,12 +162,12 @@ int launch_fused_single(pme_recip* h, const SysDesc& d_in) {
   fused_tile_counts(d, a.total);
   size_t smem = fused_smem_bytes(d);
   FusedShape shape;
-  cudaError_t e = fused_shape(a.total, smem, h->grid_cap, &shape);
+  cudaError_t e = fused_shape(a.total, smem, h->grid_cap, heavy_tiles(d), &shape);
   if (e == cudaSuccess && d.gx && shape.variant != kFusedLatency) {
     d.gx = 0;
     fused_tile_counts(d, a.total);
     smem = fused_smem_bytes(d);
-    e = fused_shape(a.total, smem, h->grid_cap, &shape);
+    e = fused_shape(a.total, smem, h->grid_cap, heavy_tiles(d), &shape);
   }
   if (e != cudaSuccess) return cuda_fail(e, "fused: launch shape (does the kernel fit on an SM?)");
   // y, z, the solve and both inverses as kx planes split over 4-CTA clusters, where the plane
@@ -740,7 +740,7 @@ int pme_batch_create(const pme_system_desc* systems, int nsys, void* stream, pme
   std::vector<size_t> off(nsys), boff(nsys);
   size_t total = 0;
   for (int i = 0; i < nsys; i++) {
-    b->st[i].setup(systems[i].nfftx, systems[i].nffty, systems[i].nfftz, systems[i].order);
+    b->st[i].setup(systems[i].nfftx, systems[i].nffty, systems[i].nfftz, systems[i].order, false);
     off[i] = total;
     total += SystemState::bytes(systems[i].nfftx, systems[i].nffty, systems[i].nfftz);
   }
@@ -817,7 +817,7 @@ int pme_batch_commit(pme_batch* b) {
   if (e == cudaSuccess) e = cudaMemcpy(b->d_prefix, prefix.data(), prefix.size() * sizeof(int), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cuda_fail(e, "batch: upload descriptors");
   b->smem = smem;
-  e = fused_shape(b->total, smem, b->grid_cap, &b->shape);
+  e = fused_shape(b->total, smem, b->grid_cap, false, &b->shape);
   if (e != cudaSuccess) return cuda_fail(e, "batch: launch shape (does the kernel fit on an SM?)");
   return PME_OK;
 }

@@ -230,12 +230,12 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a) {
 // tile per CTA in a phase.  Throughput build: at most 80 registers, 3 CTAs per SM (a few spills in
 // the largest tiles); for launches with many tiles per CTA, where the extra resident warps hide
 // more latency than the spills cost.
-__global__ void __launch_bounds__(kThreads) k_fused_lat(const __grid_constant__ FusedArgs a) { fused_body<true>(a); }
+__global__ void __launch_bounds__(kThreads, 2) k_fused_lat(const __grid_constant__ FusedArgs a) { fused_body<true>(a); }
 __global__ void __launch_bounds__(kThreads, 3) k_fused_tput(const __grid_constant__ FusedArgs a) { fused_body<false>(a); }
 // Cluster build: the latency build with the cluster plane tiles, only ever launched with clusters of
 // kClusterPlane CTAs (kept apart so that the other launches run the latency build without the
 // cluster code: compiled into one kernel, it made their evaluations 2-4 us slower).
-__global__ void __launch_bounds__(kThreads) k_fused_cl(const __grid_constant__ FusedArgs a) { fused_body<true, true>(a); }
+__global__ void __launch_bounds__(kThreads, 2) k_fused_cl(const __grid_constant__ FusedArgs a) { fused_body<true, true>(a); }
 
 // ------------------------------- staged cooperative kernel -----------------------------------
 // One reference-interface call (r2c_fft, scalar_sum, c2r_fft) as one cooperative launch over the
@@ -485,15 +485,21 @@ static cudaError_t occupancy(size_t smem, Occupancy* out) {
   return cudaSuccess;
 }
 
-cudaError_t fused_shape(const int* total, size_t smem, int grid_cap, FusedShape* out) {
+cudaError_t fused_shape(const int* total, size_t smem, int grid_cap, bool heavy, FusedShape* out) {
   Occupancy o;
   cudaError_t e = occupancy(smem, &o);
   if (e != cudaSuccess) return e;
   const int sms = o.sms, occ_lat = o.lat, occ_tput = o.tput;
   int most = 1;
   for (int p = 0; p < kPhases; p++) most = most > total[p] ? most : total[p];
-  // many tiles per CTA: more resident CTAs pay; about one: fewer registers per thread cost
-  const bool tput = occ_tput > occ_lat && most > 2 * sms * occ_lat;
+  // many tiles per CTA: more resident CTAs pay; about one: fewer registers per thread cost, unless
+  // the row blocks' tiles are long and 3 CTAs per SM take them in fewer waves (54,000 atoms,
+  // 90 x 75 x 80, order 8, 380 tiles: 188 us with 2 per SM, 167 with 3)
+  bool tput = occ_tput > occ_lat && most > 2 * sms * occ_lat;
+  if (!tput && heavy && occ_tput > occ_lat) {
+    const int wl = (total[1] + sms * occ_lat - 1) / (sms * occ_lat), wt = (total[1] + sms * occ_tput - 1) / (sms * occ_tput);
+    tput = 5 * wt < 4 * wl;   // a tile with 2 CTAs on its SM takes 0.8 of its time with 3
+  }
   out->variant = tput ? kFusedThroughput : kFusedLatency;
   out->cluster = 0;
   int grid = sms * (tput ? occ_tput : occ_lat);

@@ -197,7 +197,8 @@ struct SystemState {
            align256(4 * n * 8) + align256(kAccCount * 8) + align256(kEvCount * 8);
   }
 
-  void setup(int nx_, int ny_, int nz_, int order_) {
+  // alone: the system has launches of its own (else it shares them with a batch or a server's requests)
+  void setup(int nx_, int ny_, int nz_, int order_, bool alone = true) {
     nx = nx_; ny = ny_; nz = nz_; order = order_;
     factorize(nx, px);
     factorize(ny, py);
@@ -210,15 +211,50 @@ struct SystemState {
     tx_z = pick_cols_tile(ny, nz);
     // whole-plane tiles need one thread per line of each orientation and the plane in smem
     plane = (plane_smem_bytes(ny, nz) <= kTileSmemBudget && ny <= kThreads && nz <= kThreads) ? 1 : 0;
-    // row blocks of the fused spread + x pass: the largest square block that fits
-    for (int b = kSpreadMaxBlock; b >= 1; b--) {
-      bry = brz = b;
-      size_t need = 0;   // the order can change later (pme_set_order): size for every order
-      for (int o = 4; o <= kMaxOrder; o += 2) need = std::max(need, spread_x_smem_bytes(nx, b * b, o));
-      if (need <= kTileSmemBudget) break;
-    }
+    pick_block(alone);
     nby = (ny + bry - 1) / bry;
     nbz = (nz + brz - 1) / brz;
+  }
+
+  // Row blocks of the fused spread + x pass (and of the gather).  In launches with many systems, the
+  // largest square block that fits: fewest candidate records per contribution.  For a system alone, the
+  // block whose tiles take the least time in whole waves of resident CTAs, by a model fitted to phase
+  // traces at 0.1 atoms per grid point: a tile takes 2.5 us + 10.2 ns per candidate record (of every bin
+  // its window touches) + 0.56 ns per contribution with 3 CTAs on an SM, 0.8 of that with 2; the build
+  // with 3 per SM runs more phases (8 us); a CTA more costs the barriers 6 ns; shared memory that leaves
+  // less L1 costs up to 15% (216^3, 68 against 56 KB a CTA: gather 284 and 270 us).  Spread phase, model
+  // and trace, us: 120 x 108 x 96 order 6, blocks of 4 x 4 rows 86 and 85, 4 x 3 66 and 71, 3 x 3 76 and 77;
+  // 90 x 75 x 80 order 8, 4 x 4 57 and 55, 3 x 3 78 and 76; 216^3 order 6, 3 x 3 (of 4 x 3 and 3 x 2) 482.
+  void pick_block(bool alone) {
+    double best = 0.0;
+    bry = brz = 1;
+    for (int by = kSpreadMaxBlock; by >= 1; by--)
+      for (int bz = by; bz >= (alone ? 1 : by); bz--) {
+        size_t need = 0;   // the order can change later (pme_set_order): size for every order
+        for (int o = 4; o <= kMaxOrder; o += 2) need = std::max(need, spread_x_smem_bytes(nx, by * bz, o));
+        if (need > kTileSmemBudget) continue;
+        if (!alone) {
+          bry = brz = by;
+          return;
+        }
+        const double tiles = (double)((ny + by - 1) / by) * ((nz + bz - 1) / bz), per_row = 0.1 * nx;
+        const double cand = by * ((order - 2 + by) / by + 1) * bz * ((order - 2 + bz) / bz + 1);   // rows of the bins
+        const double tile = 2.5 + per_row * (10.2e-3 * cand + 0.56e-3 * order * order * order * by * bz);
+        const size_t smem = spread_x_smem_bytes(nx, by * bz, order) + 2048;
+        double cost = 0.0;
+        for (int ctas = 2; ctas <= 3; ctas++) {   // latency build, throughput build
+          if (ctas * smem > 227 * 1024) continue;
+          const double l1 = 1.0 + 0.15 * (double)(ctas * smem) / (227 * 1024);
+          const double c = std::ceil(tiles / (148.0 * ctas)) * tile * l1 * (ctas == 2 ? 0.8 : 1.0) + (ctas == 2 ? 0.0 : 8.0) +
+                           6e-3 * std::min(tiles, 148.0 * ctas);
+          if (cost == 0.0 || c < cost) cost = c;
+        }
+        if (best == 0.0 || cost < best) {
+          best = cost;
+          bry = by;
+          brz = bz;
+        }
+      }
   }
 
   int nbins() const { return nby * nbz; }

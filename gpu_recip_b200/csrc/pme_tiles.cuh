@@ -916,63 +916,67 @@ __device__ __forceinline__ void bin_tile(const SysDesc& d, int tile, int parity,
 // the result equals the staged spread's fixed-point grid bit for bit), then the rows are converted
 // to FP32 and x-transformed in place.
 //
-// The work is split so that every lane does the same amount: a round takes up to spread_slots(P)
-// candidates; step A tests each against the block and lists the ones that reach it (their
-// weights) and one item per (atom, block row) it covers; step B gives each lane one item at a
-// time, i.e. the P contributions of one stencil row.  The accumulator rows are P-1 points longer
-// than the grid row, so a stencil row never wraps while spreading (the overhang is folded back
-// when the rows are converted), and their stride is odd, so the rows of one atom fall in
-// different banks.
+// Each warp takes 32 candidates at a time on its own, with no CTA barrier until the tile's spreading
+// is done: their records come into the warp's part of shared memory by asynchronous copies, lane after
+// lane in consecutive 16-byte pieces (loads of whole records by single lanes touched 32 lines per
+// instruction and were half of the phase); step A tests one candidate per lane against the block and
+// lists one item per (atom, block row) it covers; step B gives each lane one item at a time, i.e. the P
+// contributions of one stencil row, weights read from the staged record.  The accumulator rows are P-1
+// points longer than the grid row, so a stencil row never wraps while spreading (the overhang is folded
+// back when the rows are converted), and their stride is odd, so the rows of one atom fall in different
+// banks.  Bound by the shared-memory atomics (two per contribution) and the latency of the records.
+// The spread + x phase, before (CTA-wide rounds of 256 or 512 candidates, their weights copied into lists,
+// three accumulator words per point) and after: 1,008,000 atoms 216^3 order 6 598 and 480 us, 54,000 atoms
+// 90 x 75 x 80 order 8 69 and 55 us, 24,000 atoms 64^3 order 6 24.1 and 19.5 us, order 4 11.5 and 11.0 us,
+// 256 systems order 4 735 and 655 us.
 // ---------------------------------------------------------------------------------------------
 constexpr int kSpreadMaxBlock = 4;                  // row-block edge limit (bry, brz)
-constexpr int kSpreadBookInts = 168;                // counters, candidate-bin offsets and bases
-// candidates per round (listed-atom slots) and the items they can produce
-__host__ __device__ constexpr int spread_slots(int order) { return order <= 4 ? 2 * kThreads : kThreads; }
-__host__ __device__ constexpr int spread_item_cap(int order) {
-  return spread_slots(order) * kSpreadMaxBlock * kSpreadMaxBlock;
-}
-
+constexpr int kSpreadBookInts = 132;                // candidate-bin offsets and bases
 __host__ __device__ inline int spread_row_stride(int nx, int order) { return (nx + order - 1) | 1; }
 __host__ __device__ inline size_t align16(size_t b) { return (b + 15) & ~(size_t)15; }
-
-// smem of the spread + x tile: 3 x 32-bit accumulators per point, twiddles, bookkeeping, then a
-// work area that holds the listed atoms and items while spreading and the FFT buffers after.
-__host__ __device__ inline size_t spread_x_smem_bytes(int nx, int rows, int order) {
-  const size_t acc = align16((size_t)rows * spread_row_stride(nx, order) * 12);
-  const size_t fft = (size_t)2 * nx * (rows + 1) * sizeof(float2);
-  const size_t lists = (size_t)spread_slots(order) * 3 * order * 4 + (size_t)spread_item_cap(order) * sizeof(unsigned int);
-  return acc + align16((size_t)nx * sizeof(float2)) + kSpreadBookInts * sizeof(int) + (fft > lists ? fft : lists);
+// Staged record: head and weights, the stride an odd number of 16-byte pieces (no bank conflicts
+// between the records of 8 lanes).
+__host__ __device__ constexpr int stage_pieces(int order) { return (4 + 3 * order + 3) / 4; }
+__host__ __device__ constexpr int stage_stride(int order) { return 4 * (stage_pieces(order) | 1); }
+// Stages per warp: two at order 4, where a tile's few candidates are mostly load latency.
+__host__ __device__ constexpr int spread_stages(int order) { return order <= 4 ? 2 : 1; }
+__host__ __device__ inline size_t spread_warp_bytes(int rows, int order) {
+  return 32 * sizeof(float) * (size_t)(spread_stages(order) * stage_stride(order) + rows);
 }
 
-// Exact int64 accumulation in shared memory with native 32-bit atomics, in one of three forms
-// chosen per tile before its first contribution.  A point receives at most one contribution per
-// candidate atom (the P stencil points of an axis are distinct), so with n candidates:
-//  split2(k): v = lo + hi 2^k, lo = v mod 2^k in [0, 2^k), hi = v >> k (signed): two sums.  The
+// smem of the spread + x tile: 2 x 32-bit accumulators per point, twiddles, bookkeeping, then a
+// work area that holds the warps' staged records and items while spreading and the FFT buffers after.
+__host__ __device__ inline size_t spread_x_smem_bytes(int nx, int rows, int order) {
+  const size_t acc = align16((size_t)rows * spread_row_stride(nx, order) * 8);
+  const size_t fft = (size_t)2 * nx * (rows + 1) * sizeof(float2);
+  const size_t work = (kThreads / 32) * spread_warp_bytes(rows, order);
+  return acc + align16((size_t)nx * sizeof(float2)) + kSpreadBookInts * sizeof(int) + (fft > work ? fft : work);
+}
+
+// Exact int64 accumulation in shared memory with native 32-bit atomics, two words per point, in one of
+// two forms chosen per tile before its first contribution.  A point receives at most one contribution
+// per candidate atom (the P stencil points of an axis are distinct), so with n candidates:
+//  split(k): v = lo + hi 2^k, lo = v mod 2^k in [0, 2^k), hi = v >> k (signed): two sums.  The
 //    lo sum stays below n 2^k <= 2^32; the hi sum's magnitude below n (|v|max / 2^k + 1), where
-//    |v| <= |q| 2^40 because every spline weight is at most 1.  k is the largest value with
+//    |v| <= |q| 2^40 M_P(P/2)^3, the cube of the spline's largest weight.  k is the largest value with
 //    n 2^k < 2^32, and the form is taken when the hi bound, from the system's max |q|, is below
-//    2^31.
-//  split3: v = p0 + p1 2^16 + p2 2^32 (p0, p1 in [0, 2^16), p2 = v >> 32): the p0 and p1 sums
-//    cannot wrap for n <= 2^16; the p2 sum may wrap, harmlessly, since only its value modulo 2^32
-//    enters the int64 result.
-//  carry: lo (u32) + hi (s32), the wrap of lo detected from the returned old value (any n).
-// Only the carry form waits for an atomic's result.  In every form the point's value is
-// s0 + s1 2^16 + s2 2^sh (s2 sign-extended; sh = k for split2, 32 otherwise) modulo 2^64.
-enum SpreadMode { kSplit2 = 0, kSplit3 = 1, kCarry = 2 };
+//    2^31 (at 2,000 candidates: |q| <= 6 at order 4, 12 at order 6, 18 at order 8).
+//  carry: lo (u32) + hi (s32), the wrap of lo detected from the returned old value (any n, any q).
+// Only the carry form waits for an atomic's result.  In either form the point's value is
+// s0 + s2 2^sh (s2 sign-extended; sh = k for split, 32 for carry) modulo 2^64.
+enum SpreadMode { kSplit = 0, kCarry = 1 };
+
+// Cube of the largest weight of the order-P spline, M_P(P/2).
+__host__ __device__ constexpr float spline_peak3(int order) {
+  return order <= 4 ? (float)(8.0 / 27.0) : (order <= 6 ? (float)(0.55 * 0.55 * 0.55)
+                                                         : (float)((151.0 / 315.0) * (151.0 / 315.0) * (151.0 / 315.0)));
+}
 
 template <int MODE>
-__device__ __forceinline__ void add_fixed(unsigned int* s0, unsigned int* s1, int* s2, int idx, long long v,
-                                          int k, unsigned int kmask) {
-  if (MODE == kSplit2) {
+__device__ __forceinline__ void add_fixed(unsigned int* s0, int* s2, int idx, long long v, int k, unsigned int kmask) {
+  if (MODE == kSplit) {
     atomicAdd(&s0[idx], (unsigned int)(unsigned long long)v & kmask);
     atomicAdd(&s2[idx], (int)(v >> k));
-  } else if (MODE == kSplit3) {
-    const unsigned long long u = (unsigned long long)v;
-    const unsigned int p0 = (unsigned int)(u & 0xffffull), p1 = (unsigned int)((u >> 16) & 0xffffull);
-    const int p2 = (int)(v >> 32);
-    atomicAdd(&s0[idx], p0);
-    atomicAdd(&s1[idx], p1);
-    if (p2 != 0) atomicAdd(&s2[idx], p2);
   } else {
     const unsigned int l = (unsigned int)(unsigned long long)v;
     const int h = (int)(v >> 32);
@@ -981,15 +985,6 @@ __device__ __forceinline__ void add_fixed(unsigned int* s0, unsigned int* s1, in
     if (h + carry != 0) atomicAdd(&s2[idx], h + carry);
   }
 }
-
-// The listed atoms of a round: w[k][slot] over spread_slots(P) slots, k < 3P: q thx, thy, thz.
-// An item is slot | b << 9 | c << 12 | (row * Lp + ix) << 15: stencil indices b (y) and c (z)
-// and the accumulator offset of the stencil row's first point.
-struct SpreadLists {
-  float* w;
-  unsigned int* items;
-  int* counters;   // [0] listed atoms, [1] items
-};
 
 // Block rows [0, nr) covered by a stencil whose first row sits at r0 in [0, n) relative to the
 // block (rows r0 .. r0+P-1, wrapped mod n), as a bitmask.
@@ -1023,110 +1018,86 @@ __device__ __forceinline__ void cand_axis(int P, int n, int br, int nb, int own,
   cnt += 1;
 }
 
-// Step A for PRE candidates per lane, their records already loaded (has[u] == false: none).
-// The lane's listed atoms and items are reserved together: one warp scan and one pair of counter
-// updates per warp.  Every lane of the warp calls it.
-template <int P, int PRE>
-__device__ __forceinline__ void spread_list_atoms(const SysDesc& d, const bool (&has)[PRE], const float4 (&head)[PRE],
-                                                  const float4 (&w4)[PRE][(rec_floats(P) - 8) / 4], int Y0, int Z0,
-                                                  int nry, int nrz, int Lp, const SpreadLists& sl) {
-  constexpr int S = spread_slots(P);
+// Step A: the items of this lane's candidate (has == false: none), head = its stencil origin, listed in
+// lane order; returns the warp's item count.  An item is lane | b << 5 | c << 8 | (row * Lp + ix) << 11:
+// the staged record, stencil indices b (y) and c (z) and the accumulator offset of the stencil row's
+// first point.  Every lane of the warp calls it.
+template <int P>
+__device__ __forceinline__ int spread_list(const SysDesc& d, bool has, float4 head, int Y0, int Z0, int nry, int nrz,
+                                           int Lp, unsigned int* items) {
   const Geom& g = d.g;
   const int lane = threadIdx.x & 31;
-  unsigned int my[PRE], mz[PRE];
-  int ry0[PRE], rz0[PRE], nrow[PRE];
-  int v = 0;   // this lane's items (low 16 bits) and listed atoms (high bits)
-#pragma unroll
-  for (int u = 0; u < PRE; u++) {
-    my[u] = mz[u] = 0u;
-    ry0[u] = rz0[u] = 0;
-    if (has[u]) {
-      ry0[u] = __float_as_int(head[u].y) - Y0;
-      if (ry0[u] < 0) ry0[u] += g.ny;
-      rz0[u] = __float_as_int(head[u].z) - Z0;
-      if (rz0[u] < 0) rz0[u] += g.nz;
-      my[u] = covered_rows(ry0[u], P, g.ny, nry);
-      mz[u] = covered_rows(rz0[u], P, g.nz, nrz);
-    }
-    nrow[u] = __popc(my[u]) * __popc(mz[u]);
-    v += nrow[u] + (nrow[u] > 0 ? 1 << 16 : 0);
+  unsigned int my = 0u, mz = 0u;
+  int ry0 = 0, rz0 = 0;
+  if (has) {
+    ry0 = __float_as_int(head.y) - Y0;
+    if (ry0 < 0) ry0 += g.ny;
+    rz0 = __float_as_int(head.z) - Z0;
+    if (rz0 < 0) rz0 += g.nz;
+    my = covered_rows(ry0, P, g.ny, nry);
+    mz = covered_rows(rz0, P, g.nz, nrz);
   }
-  int incl = v;
+  const int nrow = __popc(my) * __popc(mz);
+  int incl = nrow;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const int t = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += t;
   }
-  const int wtot = __shfl_sync(0xffffffffu, incl, 31);
-  if (wtot == 0) return;
-  int sbase = 0, ibase = 0;
-  if (lane == 0) {
-    sbase = atomicAdd(&sl.counters[0], wtot >> 16);
-    ibase = atomicAdd(&sl.counters[1], wtot & 0xffff);
-  }
-  sbase = __shfl_sync(0xffffffffu, sbase, 0);
-  ibase = __shfl_sync(0xffffffffu, ibase, 0);
-  const int excl = incl - v;
-  unsigned int slot = (unsigned int)(sbase + (excl >> 16));
-  unsigned int* it = sl.items + (ibase + (excl & 0xffff));
-#pragma unroll
-  for (int u = 0; u < PRE; u++) {
-    if (nrow[u] == 0) continue;
-    float* ws = sl.w + slot;
-#pragma unroll
-    for (int c = 0; c < 3 * P / 4; c++) {
-      ws[(4 * c) * S] = w4[u][c].x;
-      ws[(4 * c + 1) * S] = w4[u][c].y;
-      ws[(4 * c + 2) * S] = w4[u][c].z;
-      ws[(4 * c + 3) * S] = w4[u][c].w;
-    }
-    if ((3 * P) % 4 != 0) {   // P = 6: the last two weights
-      ws[(3 * P - 2) * S] = w4[u][(3 * P) / 4].x;
-      ws[(3 * P - 1) * S] = w4[u][(3 * P) / 4].y;
-    }
-    const unsigned int ix = (unsigned int)__float_as_int(head[u].x);
-    unsigned int mzz = mz[u];
-    while (mzz) {
-      const int rz = __ffs(mzz) - 1;
-      mzz &= mzz - 1;
-      int c = rz - rz0[u];
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  if (nrow > 0) {
+    unsigned int* it = items + (incl - nrow);
+    const unsigned int ix = (unsigned int)__float_as_int(head.x);
+    while (mz) {
+      const int rz = __ffs(mz) - 1;
+      mz &= mz - 1;
+      int c = rz - rz0;
       if (c < 0) c += g.nz;
-      unsigned int myy = my[u];
-      while (myy) {
-        const int ry = __ffs(myy) - 1;
-        myy &= myy - 1;
-        int b = ry - ry0[u];
+      for (unsigned int m = my; m; m &= m - 1) {
+        const int ry = __ffs(m) - 1;
+        int b = ry - ry0;
         if (b < 0) b += g.ny;
-        *it++ = slot | (unsigned int)b << 9 | (unsigned int)c << 12 | ((unsigned int)(ry + nry * rz) * Lp + ix) << 15;
+        *it++ = (unsigned int)lane | (unsigned int)b << 5 | (unsigned int)c << 8 | ((unsigned int)(ry + nry * rz) * Lp + ix) << 11;
       }
     }
-    slot++;
   }
+  return total;
 }
 
 // Step B: the P contributions of one (atom, stencil row) item per lane.
 template <int P, int MODE>
-__device__ __forceinline__ void spread_items(const SpreadLists& sl, int nitems, unsigned int* s0, unsigned int* s1,
+__device__ __forceinline__ void spread_items(const float* stage, const unsigned int* items, int nitems, unsigned int* s0,
                                              int* s2, int k2, unsigned int kmask) {
-  constexpr int S = spread_slots(P);
-  for (int j = threadIdx.x; j < nitems; j += kThreads) {
-    const unsigned int it = sl.items[j];
-    const float* ws = sl.w + (it & 511u);
-    const float ty = ws[(P + ((it >> 9) & 7u)) * S];
-    const float tz = ws[(2 * P + ((it >> 12) & 7u)) * S];
-    const int base = (int)(it >> 15);
+  for (int j = threadIdx.x & 31; j < nitems; j += 32) {
+    const unsigned int it = items[j];
+    const float* rec = stage + (it & 31u) * stage_stride(P);
+    const float ty = rec[4 + P + ((it >> 5) & 7u)];
+    const float tz = rec[4 + 2 * P + ((it >> 8) & 7u)];
+    float w[8];
+    *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(rec + 4);
+    if (P == 6) *reinterpret_cast<float2*>(w + 4) = *reinterpret_cast<const float2*>(rec + 8);
+    if (P == 8) *reinterpret_cast<float4*>(w + 4) = *reinterpret_cast<const float4*>(rec + 8);
+    const int base = (int)(it >> 11);
 #pragma unroll
-    for (int k = 0; k < P; k++)
-      add_fixed<MODE>(s0, s1, s2, base + k, fixed_contrib(ws[k * S], ty, tz), k2, kmask);
+    for (int k = 0; k < P; k++) add_fixed<MODE>(s0, s2, base + k, fixed_contrib(w[k], ty, tz), k2, kmask);
   }
+}
+
+__device__ __forceinline__ void copy_async16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned int)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_async_wait() {   // all but the last N groups have landed
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 template <int P>
 __device__ __forceinline__ void spread_x_tile(const SysDesc& d, int tile, int parity, char* smem_raw) {
   constexpr int RF = rec_floats(P);
-  constexpr int NW4 = (RF - 8) / 4;          // float4s of spreading weights
-  constexpr int S = spread_slots(P);
-  constexpr int PRE = S / kThreads;            // candidates whose records a thread loads at once
+  constexpr int NP = stage_pieces(P), RS = stage_stride(P), NST = spread_stages(P);
+  constexpr int kRound = kThreads;             // candidates the CTA's warps take per turn, 32 each
   const Geom& g = d.g;
   const FftPlan1D& plan = d.px;
   const int L = g.nx, Lp = spread_row_stride(L, P);
@@ -1137,19 +1108,16 @@ __device__ __forceinline__ void spread_x_tile(const SysDesc& d, int tile, int pa
   const int ld = rows + 1;
   const int tid = threadIdx.x;
   unsigned int* s0 = (unsigned int*)smem_raw;
-  unsigned int* s1 = s0 + (size_t)rows * Lp;
-  int* s2 = (int*)(s1 + (size_t)rows * Lp);
-  char* p = smem_raw + align16((size_t)rows * Lp * 12);
+  int* s2 = (int*)(s0 + (size_t)rows * Lp);
+  char* p = smem_raw + align16((size_t)rows * Lp * 8);
   float2* tw = (float2*)p;
   p += align16((size_t)L * sizeof(float2));
-  int* book = (int*)p;                         // [0..1] counters, [32..96] candidate-bin offsets,
-  int* coff = book + 32;                       // [100..163] their first record (in records)
-  int* cbase = book + 100;
+  int* coff = (int*)p;                         // [0..64] candidate-bin offsets,
+  int* cbase = coff + 68;                      // [0..63] their first record (in records)
   p += kSpreadBookInts * sizeof(int);
-  SpreadLists sl;
-  sl.w = (float*)p;
-  sl.items = (unsigned int*)(sl.w + (size_t)3 * P * S);
-  sl.counters = book;
+  // this warp's part of the work area: staged records, items
+  float* const stage = (float*)(p + (tid >> 5) * spread_warp_bytes(rows, P));
+  unsigned int* const items = (unsigned int*)(stage + NST * 32 * RS);
   float2* b0 = (float2*)p;                     // FFT view of the work area (after spreading)
   float2* b1 = b0 + (size_t)L * ld;
   const int nbins = d.nby * d.nbz;
@@ -1191,11 +1159,10 @@ __device__ __forceinline__ void spread_x_tile(const SysDesc& d, int tile, int pa
     coff[tid] = inc[0] - n01[0];
     coff[tid + 32] = tot0 + inc[1] - n01[1];
     if (tid == 31) coff[64] = tot0 + inc[1];
-    if (tid < 2) sl.counters[tid] = 0;
   }
   {
-    // the three accumulator arrays are one 16-byte-aligned block of 3 rows*Lp words
-    const int words = 3 * rows * Lp;
+    // the two accumulator arrays are one 16-byte-aligned block of 2 rows*Lp words
+    const int words = 2 * rows * Lp;
     uint4* z4 = (uint4*)s0;
     for (int i = tid; i < words / 4; i += kThreads) z4[i] = make_uint4(0u, 0u, 0u, 0u);
     for (int i = (words & ~3) + tid; i < words; i += kThreads) s0[i] = 0u;
@@ -1210,56 +1177,63 @@ __device__ __forceinline__ void spread_x_tile(const SysDesc& d, int tile, int pa
   const int k2 = __clz(max(ncand, 1));          // largest k with ncand 2^k < 2^32
   const unsigned int kmask = (unsigned int)((1ull << k2) - 1ull);
   // hi-sum bound in FP32 (the 1.001 covers its rounding); NaN or inf qmax fails the test
-  const float hib = (float)ncand * __fmaf_rn(qmax, ldexpf(1.001f, 40 - k2), 2.0f);
-  const int mode = hib < 2147483648.0f ? kSplit2 : (ncand <= 65536 ? kSplit3 : kCarry);
-  for (int base0 = 0; base0 < ncand; base0 += S) {
-#pragma unroll 1
-    for (int h0 = 0; h0 < S; h0 += PRE * kThreads) {
-      bool has[PRE];
-      float4 head[PRE];
-      float4 w4[PRE][NW4];
+  const float hib = (float)ncand * __fmaf_rn(qmax, ldexpf(1.001f * spline_peak3(P), 40 - k2), 2.0f);
+  const int mode = hib < 2147483648.0f ? kSplit : kCarry;
+  {
+    const int lane = tid & 31;
+    // start the copies of the 32 candidates from q0 on (their records' pieces, 32 pieces per step);
+    // true on lanes with a candidate
+    int c = 0;   // candidate bin of this lane's candidate: only ever grows
+    auto fetch = [&](int q0, float* dst) {
+      const int q = q0 + lane;
+      int r = -1;   // record in the bins, or ~(record in the overflow list)
+      if (q < total) {
+        while (q >= coff[c + 1]) c++;
+        r = cbase[c] + (q - coff[c]);
+      } else {
+        r = ~(q - total);
+      }
 #pragma unroll
-      for (int u = 0; u < PRE; u++) {
-        const int q = base0 + h0 + u * kThreads + tid;
-        const float* rec = nullptr;
-        if (q < total) {
-          int c = 0;
-          while (q >= coff[c + 1]) c++;
-          rec = d.bin_recs + ((size_t)cbase[c] + (q - coff[c])) * RF;
-        } else if (q < ncand) {
-          rec = d.ovf_recs + (size_t)(q - total) * RF;
-        }
-        has[u] = rec != nullptr;
-        if (has[u]) {
-          const float4* r4 = (const float4*)rec;
-          head[u] = __ldcg(r4);
-#pragma unroll
-          for (int c = 0; c < NW4; c++) w4[u][c] = __ldcg(r4 + 1 + c);
-        } else {
-          head[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-          for (int c = 0; c < NW4; c++) w4[u][c] = head[u];
+      for (int i = 0; i < NP; i++) {
+        const int pc = i * 32 + lane, who = pc / NP;
+        const int rr = __shfl_sync(0xffffffffu, r, who);
+        if (q0 + who < ncand) {
+          const float* src = rr >= 0 ? d.bin_recs + (size_t)rr * RF : d.ovf_recs + (size_t)(~rr) * RF;
+          copy_async16(dst + who * RS + 4 * (pc - who * NP), src + 4 * (pc - who * NP));
         }
       }
-      spread_list_atoms<P, PRE>(d, has, head, w4, Y0, Z0, nry, nrz, Lp, sl);
+      copy_async_commit();
+    };
+    int q0 = tid & ~31, st = 0;
+    if (q0 < ncand) fetch(q0, stage);
+    for (; q0 < ncand; q0 += kRound) {   // the same for all lanes of a warp
+      const float* cur = stage + st * 32 * RS;
+      if (NST == 2 && q0 + kRound < ncand) {
+        fetch(q0 + kRound, stage + (1 - st) * 32 * RS);
+        copy_async_wait<1>();
+      } else {
+        copy_async_wait<0>();
+      }
+      __syncwarp();
+      const float4 head = *reinterpret_cast<const float4*>(cur + lane * RS);
+      const int ni = spread_list<P>(d, q0 + lane < ncand, head, Y0, Z0, nry, nrz, Lp, items);
+      __syncwarp();
+      if (q0 == 0) step_mark(d, 2);
+      if (mode == kSplit) spread_items<P, kSplit>(cur, items, ni, s0, s2, k2, kmask);
+      else spread_items<P, kCarry>(cur, items, ni, s0, s2, k2, kmask);
+      __syncwarp();
+      if (NST == 1 && q0 + kRound < ncand) fetch(q0 + kRound, stage);
+      if (NST == 2) st = 1 - st;
     }
-    __syncthreads();
-    if (base0 == 0) step_mark(d, 2);
-    const int ni = sl.counters[1];
-    if (mode == kSplit2) spread_items<P, kSplit2>(sl, ni, s0, s1, s2, k2, kmask);
-    else if (mode == kSplit3) spread_items<P, kSplit3>(sl, ni, s0, s1, s2, k2, kmask);
-    else spread_items<P, kCarry>(sl, ni, s0, s1, s2, k2, kmask);
-    __syncthreads();
-    if (tid < 2) sl.counters[tid] = 0;
-    __syncthreads();
   }
+  __syncthreads();
   step_mark(d, 3);
   // the other parity's counters are cleared for the next launch by the system's first block
   if (tile == 0) {
     for (int j = tid; j < nbins; j += kThreads) d.bin_count[(1 - parity) * nbins + j] = 0;
     if (tid < 2) d.bin_meta[2 * tid + 1 - parity] = 0;   // overflow count, max |q|
   }
-  const int sh = mode == kSplit2 ? k2 : 32;
+  const int sh = mode == kSplit ? k2 : 32;
   if (tid < L) tw[tid] = tw0;
   if (tid + kThreads < L) tw[tid + kThreads] = tw1;
   // rows: r = ry + nry*rz (r < nry*nrz valid); FFT line t = r.  Point e of a row also takes the
@@ -1267,11 +1241,8 @@ __device__ __forceinline__ void spread_x_tile(const SysDesc& d, int tile, int pa
   for (int idx = tid; idx < rows * L; idx += kThreads) {
     const int t = fdiv(idx, plan.n_div), e = idx - t * L;
     const int a = t * Lp + e;
-    unsigned long long u = (unsigned long long)s0[a] + ((unsigned long long)s1[a] << 16) +
-                           ((unsigned long long)(long long)s2[a] << sh);
-    if (e < P - 1)
-      u += (unsigned long long)s0[a + L] + ((unsigned long long)s1[a + L] << 16) +
-           ((unsigned long long)(long long)s2[a + L] << sh);
+    unsigned long long u = (unsigned long long)s0[a] + ((unsigned long long)(long long)s2[a] << sh);
+    if (e < P - 1) u += (unsigned long long)s0[a + L] + ((unsigned long long)(long long)s2[a + L] << sh);
     b0[e * ld + t] = make_float2(fixed_to_float((long long)u), 0.0f);
   }
   __syncthreads();
