@@ -81,7 +81,8 @@ struct pme_batch {
   int trace_ctas = 0;
   int plane_mode = 0;   // PME_SCHED_*: AUTO and PLANES use planes where they fit
   int grid_cap = 0;
-  int line_scale = 1;   // lines per x/y/z pass tile: each system's default times this (budget permitting)
+  int line_scale = 0;   // lines per x/y/z pass tile: each system's default times this (budget permitting);
+                        // 0: the largest of 4, 2 and 1 that leaves the launch two waves of x-pass tiles
 };
 
 namespace {
@@ -240,11 +241,17 @@ void set_config(pme_recip* h, const pme_tune_config& c) {
   h->grid_cap = c.grid_ctas;
 }
 
+int sm_count(int dev) {
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 1;
+  return sms;
+}
+
 // base * scale lines per pass tile, at most limit, shrunk (not below base) until the tile's
 // shared memory (plus `extra` bytes) fits the budget.
-int scaled_lines(int L, int base, int scale, int limit, size_t extra) {
+int scaled_lines(int L, int base, int scale, int limit, size_t extra, size_t budget) {
   int t = std::min(base * scale, std::max(limit, base));
-  while (t > base && tile_smem_bytes(L, t) + extra > kTileSmemBudget) t--;
+  while (t > base && tile_smem_bytes(L, t) + extra > budget) t--;
   return t;
 }
 
@@ -798,18 +805,35 @@ int pme_batch_commit(pme_batch* b) {
   const int nsys = (int)b->desc.size();
   std::vector<int> prefix((size_t)kPhases * (nsys + 1), 0);
   size_t smem = 0;
-  for (int i = 0; i < nsys; i++) {
-    const SystemState& st = b->st[i];
-    b->desc[i].plane = (st.plane && b->plane_mode != PME_SCHED_PASSES) ? 1 : 0;
-    b->desc[i].tx_rows = scaled_lines(st.nx, st.tx_rows, b->line_scale, 64, 0);
-    b->desc[i].tx_y = scaled_lines(st.ny, st.tx_y, b->line_scale, 64, 0);
-    b->desc[i].tx_z = scaled_lines(st.nz, st.tx_z, b->line_scale, std::max(st.tx_z, st.ny),
-                                   ktab_smem_bytes(st.ny, st.nz));
-    int cnt[kPhases];
-    fused_tile_counts(b->desc[i], cnt);
-    for (int p = 0; p < kPhases; p++)
-      prefix[(size_t)p * (nsys + 1) + i + 1] = prefix[(size_t)p * (nsys + 1) + i] + cnt[p];
-    smem = std::max(smem, fused_smem_bytes(b->desc[i]));
+  // descriptors and tile prefix sums with each system's default lines times `scale`, tiles of at most
+  // `budget` bytes; returns the launch's shared memory
+  auto lay_out = [&](int scale, size_t budget) {
+    size_t most = 0;
+    for (int i = 0; i < nsys; i++) {
+      const SystemState& st = b->st[i];
+      b->desc[i].plane = (st.plane && b->plane_mode != PME_SCHED_PASSES) ? 1 : 0;
+      b->desc[i].tx_rows = scaled_lines(st.nx, st.tx_rows, scale, 64, 0, budget);
+      b->desc[i].tx_y = scaled_lines(st.ny, st.tx_y, scale, 64, 0, budget);
+      b->desc[i].tx_z = scaled_lines(st.nz, st.tx_z, scale, std::max(st.tx_z, st.ny), ktab_smem_bytes(st.ny, st.nz), budget);
+      int cnt[kPhases];
+      fused_tile_counts(b->desc[i], cnt);
+      for (int p = 0; p < kPhases; p++)
+        prefix[(size_t)p * (nsys + 1) + i + 1] = prefix[(size_t)p * (nsys + 1) + i] + cnt[p];
+      most = std::max(most, fused_smem_bytes(b->desc[i]));
+    }
+    return most;
+  };
+  if (b->line_scale > 0) {
+    smem = lay_out(b->line_scale, kTileSmemBudget);
+  } else {
+    // a 16-line tile of a short length is mostly its own latency (256 systems: 1,618 us at 1,
+    // 1,496 at 4, the x inverse 275 and 152);
+    // no more shared memory than the launch takes anyway, so that its CTAs per SM stay
+    const size_t budget = lay_out(1, kTileSmemBudget) - 2048;   // less what a tile needs beside its lines
+    for (int scale : {4, 2, 1}) {
+      smem = lay_out(scale, scale == 1 ? kTileSmemBudget : budget);
+      if (prefix[(size_t)5 * (nsys + 1) + nsys] >= 2 * 3 * sm_count(b->device)) break;
+    }
   }
   for (int p = 0; p < kPhases; p++) b->total[p] = prefix[(size_t)p * (nsys + 1) + nsys];
   cudaError_t e = cudaStreamSynchronize(b->stream);
@@ -949,12 +973,6 @@ std::vector<int> line_values(int cur) {
   std::vector<int> v = {4, 8, 16, 32};
   if (std::find(v.begin(), v.end(), cur) == v.end()) v.push_back(cur);
   return v;
-}
-
-int sm_count(int dev) {
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 1;
-  return sms;
 }
 
 }  // namespace
