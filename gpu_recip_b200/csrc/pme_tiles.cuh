@@ -1045,20 +1045,19 @@ __device__ __forceinline__ int spread_list(const SysDesc& d, bool has, float4 he
     if (lane >= o) incl += t;
   }
   const int total = __shfl_sync(0xffffffffu, incl, 31);
-  if (nrow > 0) {
-    unsigned int* it = items + (incl - nrow);
-    const unsigned int ix = (unsigned int)__float_as_int(head.x);
-    while (mz) {
-      const int rz = __ffs(mz) - 1;
-      mz &= mz - 1;
-      int c = rz - rz0;
-      if (c < 0) c += g.nz;
-      for (unsigned int m = my; m; m &= m - 1) {
-        const int ry = __ffs(m) - 1;
-        int b = ry - ry0;
-        if (b < 0) b += g.ny;
-        *it++ = (unsigned int)lane | (unsigned int)b << 5 | (unsigned int)c << 8 | ((unsigned int)(ry + nry * rz) * Lp + ix) << 11;
-      }
+  // the block's rows in order, the same for all lanes (a loop over each lane's own rows diverged)
+  unsigned int* it = items + (incl - nrow);
+  const unsigned int mine = (unsigned int)lane | (unsigned int)__float_as_int(head.x) << 11;
+#pragma unroll
+  for (int rz = 0; rz < kSpreadMaxBlock; rz++) {
+    if (rz >= nrz) break;
+    const unsigned int c = (unsigned int)(rz < rz0 ? rz - rz0 + g.nz : rz - rz0) << 8;
+    const unsigned int my_z = ((mz >> rz) & 1u) ? my : 0u;
+#pragma unroll
+    for (int ry = 0; ry < kSpreadMaxBlock; ry++) {
+      if (ry >= nry) break;
+      const unsigned int b = (unsigned int)(ry < ry0 ? ry - ry0 + g.ny : ry - ry0) << 5;
+      if ((my_z >> ry) & 1u) *it++ = mine + (b | c) + ((unsigned int)((ry + nry * rz) * Lp) << 11);
     }
   }
   return total;
