@@ -37,7 +37,7 @@ constexpr int kWarps = 4;             // warps per CTA of the pair kernel
 constexpr int kPairCtas = 5;          // its CTAs per SM
 constexpr int kCluster = 8;           // i atoms of a warp task: 4 lanes share one atom
 constexpr int kQueue = 72;            // queued candidates per i atom (at most 32 more at a time)
-constexpr int kTasksPerWarp = 3;      // pair tasks per resident warp to aim at
+constexpr int kTasksPerWarp = 5;      // pair tasks per resident warp to aim at (24,000 atoms: 5 per warp 275 us a step, 3 279, 1 308)
 constexpr int kMaxReach = 4;          // columns within the cutoff on each side, at most
 constexpr int kMaxXBins = 1024;       // x look-up entries per column, at most
 constexpr int kSquareTypes = 64;      // vdW types up to which every CTA holds the full square table
@@ -690,14 +690,15 @@ struct pme_direct {
   // per-call work space
   int cap_atoms = 0, cap_clusters = 0;
   size_t cap_cells = 0;
-  int2* d_cell_of = nullptr;  // bin and slot of every atom
-  unsigned long long* d_keys = nullptr;
-  int* d_count = nullptr;     // [atoms placed, clusters, pair-task counter, 0], then [cap_cells] counts
-  int* d_xstart = nullptr;    // [cap_cells]: per column, its x bins and its end
-  int2* d_clusters = nullptr; // first atom and column
+  char* d_atoms = nullptr;    // the block of the next six
   float4* d_pos = nullptr;
   int4* d_info = nullptr;
   ulonglong2* d_mask = nullptr;
+  unsigned long long* d_keys = nullptr;
+  int2* d_cell_of = nullptr;  // bin and slot of every atom
+  int2* d_clusters = nullptr; // first atom and column
+  int* d_count = nullptr;     // [atoms placed, clusters, pair-task counter, 0], then [cap_cells] counts
+  int* d_xstart = nullptr;    // (in d_count's block) [cap_cells]: per column, its x bins and its end
   long long* d_acc = nullptr;  // kAccN
 };
 
@@ -809,42 +810,39 @@ int ensure_ewald(pme_direct* h) {
   return PME_OK;
 }
 
+// Work space: one block for the atoms' arrays, one for the cells' (few allocations: a first call on
+// new sizes pays for each).
 int ensure_work(pme_direct* h, int n, int ncol, size_t ncell) {
-  if (n > h->cap_atoms) {
-    cudaFree(h->d_cell_of); cudaFree(h->d_keys); cudaFree(h->d_pos); cudaFree(h->d_info); cudaFree(h->d_mask);
-    h->d_cell_of = nullptr; h->d_keys = nullptr; h->d_pos = nullptr; h->d_info = nullptr; h->d_mask = nullptr;
-    h->cap_atoms = 0;
+  const int nclus = n / kCluster + std::min(n, ncol) + 1;   // every column rounds up at most once
+  if (n > h->cap_atoms || nclus > h->cap_clusters) {
+    cudaFree(h->d_atoms);
+    h->d_atoms = nullptr;
+    h->cap_atoms = h->cap_clusters = 0;
     const size_t m = (size_t)std::max(n, 1);
-    if (cudaMalloc(&h->d_cell_of, m * sizeof(int2)) != cudaSuccess ||
-        cudaMalloc(&h->d_keys, m * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc(&h->d_pos, m * sizeof(float4)) != cudaSuccess || cudaMalloc(&h->d_info, m * sizeof(int4)) != cudaSuccess ||
-        cudaMalloc(&h->d_mask, m * sizeof(ulonglong2)) != cudaSuccess) {
+    const size_t per_atom = sizeof(float4) + sizeof(int4) + sizeof(ulonglong2) + sizeof(unsigned long long) + sizeof(int2);
+    if (cudaMalloc(&h->d_atoms, m * per_atom + (size_t)nclus * sizeof(int2)) != cudaSuccess) {
       cudaGetLastError();
       return fail(PME_ENOMEM, "direct: atom work space");
     }
+    h->d_pos = reinterpret_cast<float4*>(h->d_atoms);
+    h->d_info = reinterpret_cast<int4*>(h->d_pos + m);
+    h->d_mask = reinterpret_cast<ulonglong2*>(h->d_info + m);
+    h->d_keys = reinterpret_cast<unsigned long long*>(h->d_mask + m);
+    h->d_cell_of = reinterpret_cast<int2*>(h->d_keys + m);
+    h->d_clusters = h->d_cell_of + m;
     h->cap_atoms = n;
+    h->cap_clusters = nclus;
   }
   if (ncell > h->cap_cells) {
-    cudaFree(h->d_count); cudaFree(h->d_xstart);
+    cudaFree(h->d_count);
     h->d_count = h->d_xstart = nullptr;
     h->cap_cells = 0;
-    if (cudaMalloc(&h->d_count, (ncell + 4) * sizeof(int)) != cudaSuccess ||
-        cudaMalloc(&h->d_xstart, ncell * sizeof(int)) != cudaSuccess) {
+    if (cudaMalloc(&h->d_count, (2 * ncell + 4) * sizeof(int)) != cudaSuccess) {
       cudaGetLastError();
       return fail(PME_ENOMEM, "direct: cell work space");
     }
+    h->d_xstart = h->d_count + 4 + ncell;
     h->cap_cells = ncell;
-  }
-  const int nclus = n / kCluster + std::min(n, ncol) + 1;   // every column rounds up at most once
-  if (nclus > h->cap_clusters) {
-    cudaFree(h->d_clusters);
-    h->d_clusters = nullptr;
-    h->cap_clusters = 0;
-    if (cudaMalloc(&h->d_clusters, (size_t)nclus * sizeof(int2)) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(PME_ENOMEM, "direct: clusters");
-    }
-    h->cap_clusters = nclus;
   }
   return PME_OK;
 }
@@ -907,9 +905,8 @@ int pme_direct_destroy(pme_direct* h) {
   DeviceGuard dg(h->device);
   cudaStreamSynchronize(h->stream);
   for (void* p : {(void*)h->d_vdw, (void*)h->d_vdw14, (void*)h->d_vdwtype, (void*)h->d_glob, (void*)h->d_win,
-                  (void*)h->d_far_ptr, (void*)h->d_far_idx, (void*)h->d_list14, (void*)h->d_tab, (void*)h->d_cell_of, (void*)h->d_keys,
-                  (void*)h->d_count, (void*)h->d_xstart, (void*)h->d_clusters, (void*)h->d_pos, (void*)h->d_info, (void*)h->d_mask,
-                  (void*)h->d_acc})
+                  (void*)h->d_far_ptr, (void*)h->d_far_idx, (void*)h->d_list14, (void*)h->d_tab, (void*)h->d_atoms,
+                  (void*)h->d_count, (void*)h->d_acc})
     if (p) cudaFree(p);
   delete h;
   return PME_OK;
