@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "../../include/pme_direct.h"
+#include "pme_direct_plan.h"
 #include "pme_state.h"
 
 namespace pme {
@@ -35,11 +36,8 @@ namespace direct {
 
 constexpr int kWarps = 4;             // warps per CTA of the pair kernel
 constexpr int kPairCtas = 5;          // its CTAs per SM
-constexpr int kCluster = 8;           // i atoms of a warp task: 4 lanes share one atom
 constexpr int kQueue = 72;            // queued candidates per i atom (at most 32 more at a time)
 constexpr int kTasksPerWarp = 5;      // pair tasks per resident warp to aim at (24,000 atoms: 5 per warp 275 us a step, 3 279, 1 308)
-constexpr int kMaxReach = 4;          // columns within the cutoff on each side, at most
-constexpr int kMaxXBins = 1024;       // x look-up entries per column, at most
 constexpr int kSquareTypes = 64;      // vdW types up to which every CTA holds the full square table
 constexpr int kMaxTypes = 200;        // vdW types
 constexpr float kEnergyScale = 4294967296.0f;     // 2^32
@@ -749,17 +747,9 @@ Params make_params(const pme_direct* h, int natom) {
   const double longest = std::max(h->box[0], std::max(h->box[1], h->box[2]));
   p.cut2 = p.roff2 * 1.00001f + (float)(1e-6 * longest * h->roff);
   p.marg = (float)(1e-5 + 1e-6 * longest);
-  // Columns roff / reach wide (at least, by a margin) along y and z, the width nearest to the edge of
-  // a cube of kCluster atoms at the system's density, so that a cluster is about as long as wide.
-  const double edge = std::cbrt(h->box[0] * h->box[1] * h->box[2] * kCluster / std::max(natom, 1));
-  const int reach = std::max(1, std::min(kMaxReach, (int)std::lround(h->roff / edge)));
-  for (int d = 1; d < 3; d++) {
-    p.nc[d] = std::max(1, (int)std::floor(h->box[d] * reach / (h->roff * (1.0 + 1e-5))));
-    p.reach[d - 1] = reach;
-  }
-  // x bins of about 1 A (a few atoms each), 64 MB of look-up table at most
-  const double ncol = (double)p.nc[1] * p.nc[2];
-  p.nc[0] = (int)std::max(1.0, std::min({h->box[0], (double)kMaxXBins, 16.0e6 / ncol}));
+  const Columns c = plan_columns(h->box, h->roff, natom);
+  for (int d = 0; d < 3; d++) p.nc[d] = c.nc[d];
+  p.reach[0] = p.reach[1] = c.reach;
   p.tab = h->d_tab;
   p.tab_n = h->elec_model == PME_ELEC_NONE ? 0 : h->tab_n;
   return p;
@@ -1074,7 +1064,7 @@ int pme_direct_calc_force(pme_direct* h, const void* xyzq, int ncoord, int calc_
   if (int rc = ensure_ewald(h)) return rc;
   Params p = make_params(h, ncoord);
   if (h->vdw_model == PME_VDW_NONE) p.ntype = 0;
-  const int ncol = p.nc[1] * p.nc[2];
+  const int ncol = p.nc[1] * p.nc[2];   // both bounded by plan_columns
   const size_t ncell = (size_t)ncol * (p.nc[0] + 1);
   if (int rc = ensure_work(h, ncoord, ncol, ncell)) return rc;
   cudaStream_t s = h->stream;

@@ -1,0 +1,46 @@
+"""The direct-space engine's host-side choices (csrc/pme_direct_plan.h), compiled with the undefined
+behaviour sanitizer and checked without a GPU."""
+import itertools
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("plan") / "direct_plan")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fsanitize=undefined,float-cast-overflow", "-fno-sanitize-recover=all",
+                    "-I", os.path.join(ROOT, "gpu_recip_b200", "csrc"), os.path.join(ROOT, "tests", "cpp", "direct_plan.cpp"),
+                    "-o", exe], check=True)
+
+    def run(what, lines):
+        text = "".join(" ".join(repr(v) for v in line) + "\n" for line in lines)
+        r = subprocess.run([exe, what], input=text, capture_output=True, text=True)
+        assert r.returncode == 0, r.stderr
+        return np.array([[float(v) for v in line.split()] for line in r.stdout.splitlines()])
+    return run
+
+
+def test_columns_stay_within_their_tables(plan):
+    """Any accepted box and cutoff (at most half the shortest edge): indices that fit, no offset that
+    wraps twice, no pair within the cutoff beyond the columns in reach."""
+    edges = [0.5, 18.0, 62.1, 500.0, 1.0e4, 1.0e6]
+    cases = [(*b, f * min(b), n) for b in itertools.product(edges, repeat=3)
+             for f in (0.5, 0.49999, 0.145, 0.02, 2e-5, 1e-9, 1e-30) for n in (1, 24000, 10 ** 6, 10 ** 9)]
+    out = plan("columns", cases)
+    box, roff = np.array([c[:3] for c in cases]), np.array([c[3] for c in cases])
+    nx, ncol, reach, cells = out[:, 0], out[:, 1:3], out[:, 3:4], out[:, 4]
+    assert (nx >= 1).all() and (nx <= 1024).all() and (ncol.prod(1) <= 2 ** 22).all()
+    assert (cells == ncol.prod(1) * (nx + 1)).all() and (cells <= 16.0e6 + 2 ** 22).all()
+    assert (reach >= 1).all() and (reach <= 4).all() and (ncol >= reach).all()
+    assert (reach * box[:, 1:] / ncol >= roff[:, None] * 1.00001 * (1 - 1e-12)).all()
+
+
+def test_columns_of_usual_systems(plan):
+    """24,000 and 192,000 atoms of water at 9 A, and a cutoff of half the box."""
+    out = plan("columns", [(62.1, 62.1, 62.1, 9.0, 24000), (124.2, 124.2, 124.2, 9.0, 192000), (18.0, 18.0, 18.0, 9.0, 600)])
+    assert out[:, :4].tolist() == [[62, 13, 13, 2], [124, 27, 27, 2], [18, 3, 3, 2]]
