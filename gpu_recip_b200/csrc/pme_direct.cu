@@ -29,6 +29,7 @@
 
 #include "../../include/pme_direct.h"
 #include "pme_direct_plan.h"
+#include "pme_direct_sum.h"
 #include "pme_state.h"
 
 namespace pme {
@@ -321,7 +322,6 @@ __global__ void __launch_bounds__(kWarps * 32, kPairCtas) k_direct_pairs(
     for (int k = threadIdx.x; k < p.ntype * p.ntype; k += blockDim.x) sh_vdw[k] = vdw_c6c12(vdwp, k / p.ntype, k % p.ntype);
   __syncthreads();
   const unsigned kFull = 0xffffffffu;
-  const double kMagic = 6755399441055744.0;   // 1.5 * 2^52: the low bits of v + kMagic hold rint(v)
   const int kNoImage = 1 | 1 << 2 | 1 << 4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & 3;
   const unsigned below = (1u << lane) - 1u;
@@ -367,8 +367,8 @@ __global__ void __launch_bounds__(kWarps * 32, kPairCtas) k_direct_pairs(
         hi[c] = fmaxf(hi[c], __shfl_xor_sync(kFull, hi[c], d));
       }
     __syncwarp();
-    long long ax = 0, ay = 0, az = 0;   // force sums at 2^40, each term plus the bits of kMagic
-    int terms = 0;                      // terms added
+    RoundedSum ax, ay, az;              // force sums at 2^40
+    int terms = 0;                      // terms added by add_rounded
     int cnt[kCluster];                  // queued hits per atom (the same on every lane)
 #pragma unroll
     for (int q = 0; q < kCluster; q++) cnt[q] = 0;
@@ -522,23 +522,23 @@ __global__ void __launch_bounds__(kWarps * 32, kPairCtas) k_direct_pairs(
         double fx = f * dx, fy = f * dy, fz = f * dz;
         // rint(v 2^40) by one addition where |v| 2^40 < 2^51: the integer is the sum's low bits
         if (!slow) {
-          ax += __double_as_longlong(__fma_rn(fx, 1099511627776.0, kMagic));
-          ay += __double_as_longlong(__fma_rn(fy, 1099511627776.0, kMagic));
-          az += __double_as_longlong(__fma_rn(fz, 1099511627776.0, kMagic));
+          ax.add_rounded(__fma_rn(fx, 1099511627776.0, kRoundMagic));
+          ay.add_rounded(__fma_rn(fy, 1099511627776.0, kRoundMagic));
+          az.add_rounded(__fma_rn(fz, 1099511627776.0, kRoundMagic));
           terms++;
           if (EV) {
-            const long long bits = __double_as_longlong(kMagic);
-            ev += __double_as_longlong(__fma_rn(uv, 4294967296.0, kMagic)) - bits;
-            ee += __double_as_longlong(__fma_rn(ue, 4294967296.0, kMagic)) - bits;
+            const long long bits = __double_as_longlong(kRoundMagic);
+            ev += __double_as_longlong(__fma_rn(uv, 4294967296.0, kRoundMagic)) - bits;
+            ee += __double_as_longlong(__fma_rn(ue, 4294967296.0, kRoundMagic)) - bits;
           }
         } else {   // outside the table, or a large (or non-finite) term: rounded by conversion
           f = pair_terms_f64(r2, qq, cc, p, uv, ue);
           fx = f * dx;
           fy = f * dy;
           fz = f * dz;
-          ax += __double2ll_rn(fx * 1099511627776.0);
-          ay += __double2ll_rn(fy * 1099511627776.0);
-          az += __double2ll_rn(fz * 1099511627776.0);
+          ax.add(__double2ll_rn(fx * 1099511627776.0));
+          ay.add(__double2ll_rn(fy * 1099511627776.0));
+          az.add(__double2ll_rn(fz * 1099511627776.0));
           if (EV) {
             ev += __double2ll_rn(uv * 4294967296.0);
             ee += __double2ll_rn(ue * 4294967296.0);
@@ -555,18 +555,15 @@ __global__ void __launch_bounds__(kWarps * 32, kPairCtas) k_direct_pairs(
       if (last) break;
     }
     // the 4 lanes of an atom join their sums; one lane per component adds it to the force array
-    const long long base = (long long)terms * __double_as_longlong(kMagic);
-    ax -= base; ay -= base; az -= base;
+    unsigned long long fx = ax.total(terms), fy = ay.total(terms), fz = az.total(terms);
 #pragma unroll
     for (int d = 1; d < 4; d <<= 1) {
-      ax += __shfl_xor_sync(kFull, ax, d);
-      ay += __shfl_xor_sync(kFull, ay, d);
-      az += __shfl_xor_sync(kFull, az, d);
+      fx += __shfl_xor_sync(kFull, fx, d);
+      fy += __shfl_xor_sync(kFull, fy, d);
+      fz += __shfl_xor_sync(kFull, fz, d);
     }
-    if (act && sub < 3) {
-      const long long v = sub == 0 ? ax : (sub == 1 ? ay : az);
-      atomicAdd((unsigned long long*)&force[ii.z + (size_t)sub * stride], (unsigned long long)v);
-    }
+    if (act && sub < 3)
+      atomicAdd((unsigned long long*)&force[ii.z + (size_t)sub * stride], sub == 0 ? fx : (sub == 1 ? fy : fz));
     if (EV) {
       wv[0] += __double2ll_rn(w0 * 4294967296.0); wv[1] += __double2ll_rn(w1 * 4294967296.0);
       wv[2] += __double2ll_rn(w2 * 4294967296.0); wv[3] += __double2ll_rn(w3 * 4294967296.0);

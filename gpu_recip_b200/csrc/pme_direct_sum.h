@@ -1,0 +1,41 @@
+// pme_direct_sum.h -- exact sums of the pair kernel's force terms, each rounded once to 2^-40.  Plain C++
+// beside CUDA, so that the arithmetic can be checked without a GPU.
+#pragma once
+
+#include <cstring>
+
+#ifdef __CUDACC__
+#define PME_SUM_FN __host__ __device__ __forceinline__
+#else
+#define PME_SUM_FN inline
+#endif
+
+namespace pme {
+namespace direct {
+
+constexpr double kRoundMagic = 6755399441055744.0;   // 1.5 * 2^52: the low bits of v + kRoundMagic hold rint(v)
+
+PME_SUM_FN unsigned long long bits_of(double v) {
+#ifdef __CUDA_ARCH__
+  return (unsigned long long)__double_as_longlong(v);
+#else
+  unsigned long long u;
+  std::memcpy(&u, &v, sizeof(u));
+  return u;
+#endif
+}
+
+// Sum of integers rint(v), |v| < 2^51, given as v + kRoundMagic: every term adds the bits of kRoundMagic
+// too, which are taken off once at the end.  All of it modulo 2^64, where the wrap is defined; the result
+// is the sum's two's complement.
+struct RoundedSum {
+  unsigned long long bits = 0ull;
+  PME_SUM_FN void add_rounded(double v_plus_magic) { bits += bits_of(v_plus_magic); }
+  PME_SUM_FN void add(long long v) { bits += (unsigned long long)v; }
+  PME_SUM_FN unsigned long long total(int rounded_terms) const {
+    return bits - (unsigned long long)rounded_terms * bits_of(kRoundMagic);
+  }
+};
+
+}  // namespace direct
+}  // namespace pme

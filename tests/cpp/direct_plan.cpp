@@ -1,8 +1,10 @@
-// Host-side choices of the direct-space engine, printed for tests/test_direct_plan.py (no GPU).
+// Host-side choices and sums of the direct-space engine, printed for tests/test_direct_plan.py (no GPU).
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 
 #include "pme_direct_plan.h"
+#include "pme_direct_sum.h"
 
 using namespace pme::direct;
 
@@ -17,7 +19,26 @@ static int columns() {
   return 0;
 }
 
+// terms per line of stdin -> their sum at 2^40 by RoundedSum after every one; terms of 2^10 and more go
+// the way of the kernel's large ones
+static int sums() {
+  double v;
+  RoundedSum a;
+  int terms = 0;
+  while (std::scanf("%lf", &v) == 1) {
+    if (std::fabs(v) < 1024.0) {
+      a.add_rounded(std::fma(v, 1099511627776.0, kRoundMagic));
+      terms++;
+    } else {
+      a.add(std::llrint(v * 1099511627776.0));
+    }
+    std::printf("%lld\n", (long long)a.total(terms));
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   if (argc == 2 && !std::strcmp(argv[1], "columns")) return columns();
+  if (argc == 2 && !std::strcmp(argv[1], "sums")) return sums();
   return 1;
 }

@@ -1,5 +1,5 @@
-"""The direct-space engine's host-side choices (csrc/pme_direct_plan.h), compiled with the undefined
-behaviour sanitizer and checked without a GPU."""
+"""The direct-space engine's host-side choices (csrc/pme_direct_plan.h) and exact sums
+(csrc/pme_direct_sum.h), compiled with the undefined behaviour sanitizer and checked without a GPU."""
 import itertools
 import os
 import subprocess
@@ -21,7 +21,7 @@ def plan(tmp_path_factory):
         text = "".join(" ".join(repr(v) for v in line) + "\n" for line in lines)
         r = subprocess.run([exe, what], input=text, capture_output=True, text=True)
         assert r.returncode == 0, r.stderr
-        return np.array([[float(v) for v in line.split()] for line in r.stdout.splitlines()])
+        return [line.split() for line in r.stdout.splitlines()]
     return run
 
 
@@ -31,7 +31,7 @@ def test_columns_stay_within_their_tables(plan):
     edges = [0.5, 18.0, 62.1, 500.0, 1.0e4, 1.0e6]
     cases = [(*b, f * min(b), n) for b in itertools.product(edges, repeat=3)
              for f in (0.5, 0.49999, 0.145, 0.02, 2e-5, 1e-9, 1e-30) for n in (1, 24000, 10 ** 6, 10 ** 9)]
-    out = plan("columns", cases)
+    out = np.array(plan("columns", cases), float)
     box, roff = np.array([c[:3] for c in cases]), np.array([c[3] for c in cases])
     nx, ncol, reach, cells = out[:, 0], out[:, 1:3], out[:, 3:4], out[:, 4]
     assert (nx >= 1).all() and (nx <= 1024).all() and (ncol.prod(1) <= 2 ** 22).all()
@@ -43,4 +43,15 @@ def test_columns_stay_within_their_tables(plan):
 def test_columns_of_usual_systems(plan):
     """24,000 and 192,000 atoms of water at 9 A, and a cutoff of half the box."""
     out = plan("columns", [(62.1, 62.1, 62.1, 9.0, 24000), (124.2, 124.2, 124.2, 9.0, 192000), (18.0, 18.0, 18.0, 9.0, 600)])
-    assert out[:, :4].tolist() == [[62, 13, 13, 2], [124, 27, 27, 2], [18, 3, 3, 2]]
+    assert [[int(v) for v in row[:4]] for row in out] == [[62, 13, 13, 2], [124, 27, 27, 2], [18, 3, 3, 2]]
+
+
+def test_force_sums_are_exact(plan):
+    """Sums of terms rounded to 2^-40: exact at every step, in defined arithmetic, small and large terms."""
+    rng = np.random.default_rng(3)
+    v = np.concatenate([rng.normal(0.0, 300.0, 400).clip(-1023.9, 1023.9), [1023.999, -1023.999, 0.0, -0.0, 0.5 ** 41, -0.5 ** 41],
+                        rng.normal(0.0, 4000.0, 200)])
+    rng.shuffle(v)
+    got = [int(row[0]) for row in plan("sums", [(float(x),) for x in v])]
+    want = np.cumsum([int(np.rint(x * 2.0 ** 40)) for x in v], dtype=object)
+    assert got == list(want)
