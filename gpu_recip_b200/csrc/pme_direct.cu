@@ -834,6 +834,20 @@ int ensure_work(pme_direct* h, int n, int ncol, size_t ncell) {
   return PME_OK;
 }
 
+// Every build of the pair kernel may take all of the device's shared memory per CTA.  The limit belongs
+// to the process, so it is only ever set to this one value: a handle that set it to what its own tables
+// need could lower it between another thread's choice and launch.
+cudaError_t configure_pair_kernels(int device) {
+  int most = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  for (auto kern : {k_direct_pairs<true, true>, k_direct_pairs<false, true>, k_direct_pairs<true, false>, k_direct_pairs<false, false>}) {
+    cudaFuncAttributes fa;
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kern);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes);
+  }
+  return e;
+}
+
 // Exclusion windows of n atoms with no exclusions but themselves.
 int self_exclusions(pme_direct* h, int n) {
   std::vector<ulonglong2> win((size_t)n, make_ulonglong2(0ull, 1ull));   // bit 64: offset 0
@@ -875,6 +889,7 @@ int pme_direct_create(void* stream, pme_direct** out) {
   if (!h) return fail(PME_ENOMEM, "host allocation failed");
   cudaError_t e = cudaGetDevice(&h->device);
   h->stream = (cudaStream_t)stream;
+  if (e == cudaSuccess) e = configure_pair_kernels(h->device);
   if (e == cudaSuccess && cudaMalloc(&h->d_acc, kAccN * sizeof(long long)) != cudaSuccess) e = cudaErrorMemoryAllocation;
   if (e == cudaSuccess) e = cudaMemset(h->d_acc, 0, kAccN * sizeof(long long));
   if (e != cudaSuccess) {
@@ -1082,8 +1097,6 @@ int pme_direct_calc_force(pme_direct* h, const void* xyzq, int ncoord, int calc_
                         : (ev ? k_direct_pairs<true, false> : k_direct_pairs<false, false>);
   const size_t smem = (size_t)p.tab_n * (ev ? 2 : 1) * sizeof(double4) +
                       (size_t)(p.square ? p.ntype * p.ntype : 0) * sizeof(float2);
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 48 * 1024));
-  if (e != cudaSuccess) return cuda_fail(e, "direct: shared memory");
   // one wave of resident CTAs; their warps draw the tasks from a counter.  Few clusters: more tasks
   // each, so that the last ones to finish are short
   int occ = 1;

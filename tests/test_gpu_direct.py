@@ -276,3 +276,45 @@ def test_direct_cluster_edges_match_oracle(cuda, oracle, box, n, roff, ntype, ka
     assert np.array_equal(fi, fi2) and e == e2 and np.array_equal(vir, vir2)
     assert np.array_equal(fi, fz.view(3, stride)[:, :n].T.cpu().numpy())
     dr.close()
+
+
+def test_handles_of_unlike_tables_in_two_threads(cuda):
+    """A handle with 64 vdW types and one with two, each in a thread with its own stream: neither's
+    launches depend on the shared memory that the other's tables take."""
+    import threading
+    from gpu_recip_b200.direct import CudaPMEDirectForce
+    d = _lattice()
+    n = d["xyzq"].shape[0]
+    failed, out = [], {}
+
+    def work(ntype):
+        try:
+            stream = cuda.cuda.Stream()
+            dr = CudaPMEDirectForce(stream)
+            dr.setup(24.0, 24.0, 24.0, 0.35, 12.0, 10.0, 1.0)
+            dr.set_vdwparam(np.ones(ntype * (ntype + 1), np.float32))
+            dr.set_vdwtype(np.arange(n, dtype=np.int32) % ntype)
+            with cuda.cuda.stream(stream):
+                x = cuda.from_numpy(np.ascontiguousarray(d["xyzq"], dtype=np.float32)).cuda()
+                f = cuda.zeros(3 * n, dtype=cuda.int64, device="cuda")
+                for _ in range(1500):
+                    f.zero_()
+                    dr.calc_force(x, n, True, True, n, f)
+                stream.synchronize()
+                out[ntype] = f.cpu().numpy(), dr
+        except Exception as e:   # raised again by the assertion below
+            failed.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in (64, 2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+    for ntype, (f, dr) in out.items():
+        g = cuda.zeros(3 * n, dtype=cuda.int64, device="cuda")
+        cuda.cuda.synchronize()
+        dr.calc_force(cuda.from_numpy(np.ascontiguousarray(d["xyzq"], dtype=np.float32)).cuda(), n, True, True, n, g)
+        cuda.cuda.synchronize()
+        assert np.array_equal(f, g.cpu().numpy())
+        dr.close()
