@@ -713,7 +713,7 @@ cudaError_t upload(T** dst, const T* src, size_t n, cudaStream_t s) {
   return e;
 }
 
-Params make_params(const pme_direct* h, int natom) {
+Params make_params(const pme_direct* h) {
   Params p;
   std::memset(&p, 0, sizeof(p));
   for (int d = 0; d < 3; d++) {
@@ -744,9 +744,6 @@ Params make_params(const pme_direct* h, int natom) {
   const double longest = std::max(h->box[0], std::max(h->box[1], h->box[2]));
   p.cut2 = p.roff2 * 1.00001f + (float)(1e-6 * longest * h->roff);
   p.marg = (float)(1e-5 + 1e-6 * longest);
-  const Columns c = plan_columns(h->box, h->roff, natom);
-  for (int d = 0; d < 3; d++) p.nc[d] = c.nc[d];
-  p.reach[0] = p.reach[1] = c.reach;
   p.tab = h->d_tab;
   p.tab_n = h->elec_model == PME_ELEC_NONE ? 0 : h->tab_n;
   return p;
@@ -797,10 +794,13 @@ int ensure_ewald(pme_direct* h) {
   return PME_OK;
 }
 
-// Work space: one block for the atoms' arrays, one for the cells' (few allocations: a first call on
-// new sizes pays for each).
-int ensure_work(pme_direct* h, int n, int ncol, size_t ncell) {
-  const int nclus = n / kCluster + std::min(n, ncol) + 1;   // every column rounds up at most once
+// Work space for n atoms in `c`: one block for the atoms' arrays, one for the cells' (few allocations: a
+// first call on new sizes pays for each), with room for a somewhat larger box.
+int ensure_work(pme_direct* h, int n, const Columns& c) {
+  if (n <= h->cap_atoms && most_clusters(n, c) <= h->cap_clusters && c.cells() <= h->cap_cells) return PME_OK;
+  const Columns room = room_columns(h->box, h->roff, n);
+  const int nclus = std::max(most_clusters(n, c), most_clusters(n, room));
+  const size_t ncell = std::max(c.cells(), room.cells());
   if (n > h->cap_atoms || nclus > h->cap_clusters) {
     cudaFree(h->d_atoms);
     h->d_atoms = nullptr;
@@ -1074,11 +1074,14 @@ int pme_direct_calc_force(pme_direct* h, const void* xyzq, int ncoord, int calc_
     h->max_type = 0;
   }
   if (int rc = ensure_ewald(h)) return rc;
-  Params p = make_params(h, ncoord);
+  Params p = make_params(h);
   if (h->vdw_model == PME_VDW_NONE) p.ntype = 0;
-  const int ncol = p.nc[1] * p.nc[2];   // both bounded by plan_columns
-  const size_t ncell = (size_t)ncol * (p.nc[0] + 1);
-  if (int rc = ensure_work(h, ncoord, ncol, ncell)) return rc;
+  const Columns cols = plan_columns(h->box, h->roff, ncoord);
+  for (int d = 0; d < 3; d++) p.nc[d] = cols.nc[d];
+  p.reach[0] = p.reach[1] = cols.reach;
+  const int ncol = cols.count();
+  const size_t ncell = cols.cells();
+  if (int rc = ensure_work(h, ncoord, cols)) return rc;
   cudaStream_t s = h->stream;
   int* const count = h->d_count + 4;
   cudaError_t e = cudaMemsetAsync(h->d_count, 0, (ncell + 4) * sizeof(int), s);
@@ -1105,7 +1108,7 @@ int pme_direct_calc_force(pme_direct* h, const void* xyzq, int ncoord, int calc_
   const long long warps = (long long)sms * std::max(occ, 1) * kWarps;
   const long long nclus = ncoord / kCluster + 1;
   p.slices = (int)std::max<long long>(1, std::min<long long>((kTasksPerWarp * warps + nclus - 1) / nclus, 2 * p.reach[1] + 1));
-  const long long tasks = (long long)h->cap_clusters * p.slices;
+  const long long tasks = (long long)most_clusters(ncoord, cols) * p.slices;
   const int pg = (int)std::max<long long>(1, std::min<long long>((tasks + kWarps - 1) / kWarps, warps / kWarps));
   kern<<<pg, kWarps * 32, smem, s>>>(p, h->d_count + 1, h->d_clusters, h->d_xstart, h->d_pos, h->d_info, h->d_mask,
                                      h->d_far_ptr, h->d_far_idx, h->d_vdw, calc_energy ? 1 : 0, calc_virial ? 1 : 0,
@@ -1130,7 +1133,7 @@ int pme_direct_calc_14_force(pme_direct* h, const void* xyzq, int calc_energy, i
     if (h->max_type >= h->ntype14) return fail(PME_EINVAL, "direct 14: a vdW type is beyond the 1-4 table");
   }
   DeviceGuard dg(h->device);
-  const Params p = make_params(h, 0);
+  const Params p = make_params(h);
   k_direct_14<<<(h->n14 + 255) / 256, 256, 0, h->stream>>>(p, h->d_list14, h->n14, (const float4*)xyzq, h->d_vdwtype,
                                                            h->d_vdw14, calc_energy ? 1 : 0, calc_virial ? 1 : 0,
                                                            stride, force, h->d_acc);

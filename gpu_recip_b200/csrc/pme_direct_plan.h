@@ -45,5 +45,16 @@ inline Columns plan_columns(const double* box, double roff, int natom) {
   return c;
 }
 
+// Clusters that n atoms make at most: every column rounds up once.
+inline int most_clusters(int n, const Columns& c) { return n / kCluster + std::min(n, c.count()) + 1; }
+
+// Columns of a box 5% longer along every edge at the same density: room for a box that breathes (constant
+// pressure) without new work space at each new maximum, where a column more along an axis can be a
+// quarter more cells.
+inline Columns room_columns(const double* box, double roff, int natom) {
+  const double f = 1.05, b[3] = {f * box[0], f * box[1], f * box[2]};
+  return plan_columns(b, roff, (int)std::min(2147483647.0, std::ceil(f * f * f * natom)));
+}
+
 }  // namespace direct
 }  // namespace pme

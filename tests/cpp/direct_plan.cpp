@@ -8,13 +8,14 @@
 
 using namespace pme::direct;
 
-// box and cutoff and atom count per line of stdin -> x bins, columns along y and z, reach, cells
+// box and cutoff and atom count per line of stdin -> x bins, columns along y and z, reach, cells;
+// cells and columns with room for a longer box
 static int columns() {
   double b[3], roff;
   int n;
   while (std::scanf("%lf %lf %lf %lf %d", &b[0], &b[1], &b[2], &roff, &n) == 5) {
-    const Columns c = plan_columns(b, roff, n);
-    std::printf("%d %d %d %d %zu\n", c.nc[0], c.nc[1], c.nc[2], c.reach, c.cells());
+    const Columns c = plan_columns(b, roff, n), m = room_columns(b, roff, n);
+    std::printf("%d %d %d %d %zu %zu %d\n", c.nc[0], c.nc[1], c.nc[2], c.reach, c.cells(), m.cells(), m.count());
   }
   return 0;
 }

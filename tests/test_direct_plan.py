@@ -46,6 +46,19 @@ def test_columns_of_usual_systems(plan):
     assert [[int(v) for v in row[:4]] for row in out] == [[62, 13, 13, 2], [124, 27, 27, 2], [18, 3, 3, 2]]
 
 
+def test_room_for_a_longer_box(plan):
+    """Edges up to 5% longer take no more cells than were made room for, whatever the box and density."""
+    rng = np.random.default_rng(5)
+    cases = []
+    for _ in range(300):
+        box = np.exp(rng.uniform(np.log(19.0), np.log(300.0), 3))
+        n = int(np.exp(rng.uniform(np.log(1e-5), np.log(0.2))) * box.prod()) + 1
+        cases += [(*(s * box).tolist(), 9.0, n) for s in (1.0, 1.003, 1.01, 1.02, 1.03, 1.04, 1.0499)]
+    out = np.array(plan("columns", cases), float).reshape(-1, 7, 7)
+    room, cells, columns = out[:, 0, 5], out[:, :, 4], out[:, :, 1] * out[:, :, 2]
+    assert (cells <= room[:, None]).all() and (columns <= out[:, 0, 6][:, None]).all()
+
+
 def test_force_sums_are_exact(plan):
     """Sums of terms rounded to 2^-40: exact at every step, in defined arithmetic, small and large terms."""
     rng = np.random.default_rng(3)

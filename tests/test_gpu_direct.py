@@ -278,6 +278,39 @@ def test_direct_cluster_edges_match_oracle(cuda, oracle, box, n, roff, ntype, ka
     dr.close()
 
 
+@pytest.mark.parametrize("box", [(40.0, 40.0, 40.0), (62.0, 70.0, 55.0)])
+def test_breathing_box_needs_no_new_work_space(cuda, box):
+    """Edges up to 4% longer than at the first call: calc_force allocates nothing (an allocation ends a
+    stream capture) and gives what a new handle gives for that box."""
+    from gpu_recip_b200.direct import CudaPMEDirectForce, EWALD, VDW_NONE
+    n = int(0.1 * np.prod(box))
+    rng = np.random.default_rng(11)
+    stream = cuda.cuda.Stream()
+    with cuda.cuda.stream(stream):
+        x = cuda.from_numpy(np.concatenate([rng.random((n, 3)) * box, rng.normal(0.0, 0.4, (n, 1))], 1).astype(np.float32)).cuda()
+        f, g = (cuda.zeros(3 * n, dtype=cuda.int64, device="cuda") for _ in range(2))
+        dr = CudaPMEDirectForce(stream)
+        dr.setup(*box, 0.33, 9.0, 7.5, 1.0, VDW_NONE, EWALD)
+        dr.calc_force(x, n, False, False, n, f)
+    stream.synchronize()
+    for scale in (1.01, 1.025, 1.04):
+        dr.set_box_size(*(scale * b for b in box))
+        graph = cuda.cuda.CUDAGraph()
+        with cuda.cuda.graph(graph, stream=stream):
+            dr.calc_force(x, n, False, False, n, f)
+        f.zero_()
+        g.zero_()
+        graph.replay()
+        new = CudaPMEDirectForce()
+        new.setup(*(scale * b for b in box), 0.33, 9.0, 7.5, 1.0, VDW_NONE, EWALD)
+        new.calc_force(x, n, False, False, n, g)
+        cuda.cuda.synchronize()
+        assert cuda.equal(f, g) and f.abs().max() > 0
+        del graph
+        new.close()
+    dr.close()
+
+
 def test_handles_of_unlike_tables_in_two_threads(cuda):
     """A handle with 64 vdW types and one with two, each in a thread with its own stream: neither's
     launches depend on the shared memory that the other's tables take."""
