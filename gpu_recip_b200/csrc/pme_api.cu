@@ -156,20 +156,17 @@ int launch_fused_single(pme_recip* h, const SysDesc& d_in) {
   d.bin_atoms = (d.natom + kThreads - 1) / kThreads < sms ? kThreads / 2 : kThreads;
   // inverse x pass inside the gather tiles where its rows fit in the shared memory the other
   // phases already take (so that the launch keeps its CTAs per SM)
-  // (latency build only: the throughput build, for launches with many tiles per CTA, keeps the
-  // separate phase and is compiled without the fused variant)
-  d.gx = 0;
-  if (h->x_gather == PME_XGATHER_AUTO && gx_smem_bytes(d.g.nx, d.bry, d.brz, d.order) <= fused_smem_bytes(d)) d.gx = 1;
+  // (latency build only: the throughput build keeps the separate phase and is compiled without the
+  // fused variant) and its 2 CTAs per SM take all gather tiles in one wave: the rows of the halo are
+  // transformed again by every tile, 2 to 4 times the phase's work, which a second wave does not hide
+  // (order 4, fused and separate: 40^3, 196 tiles, 45.6 and 46.3 us; 64^3, 256, 48.3 and 48.2; 72^3,
+  // 324, 85.4 and 81.3; 576 tiles 94.4 and 85.8)
+  d.gx = h->x_gather == PME_XGATHER_AUTO && h->st.ctas <= 2 && tiles_blocks(d) <= 2 * sms &&
+                 gx_smem_bytes(d.g.nx, d.bry, d.brz, d.order) <= fused_smem_bytes(d) ? 1 : 0;
   fused_tile_counts(d, a.total);
   size_t smem = fused_smem_bytes(d);
   FusedShape shape;
-  cudaError_t e = fused_shape(a.total, smem, h->grid_cap, heavy_tiles(d), &shape);
-  if (e == cudaSuccess && d.gx && shape.variant != kFusedLatency) {
-    d.gx = 0;
-    fused_tile_counts(d, a.total);
-    smem = fused_smem_bytes(d);
-    e = fused_shape(a.total, smem, h->grid_cap, heavy_tiles(d), &shape);
-  }
+  cudaError_t e = fused_shape(a.total, smem, h->grid_cap, h->st.ctas, &shape);
   if (e != cudaSuccess) return cuda_fail(e, "fused: launch shape (does the kernel fit on an SM?)");
   // y, z, the solve and both inverses as kx planes split over 4-CTA clusters, where the plane
   // count alone would leave most SMs idle (latency build, orthorhombic, line counts divisible);
@@ -283,7 +280,7 @@ int pme_create(int nfftx, int nffty, int nfftz, int order, int fft_type, int nno
   if (e != cudaSuccess) { delete h; return cuda_fail(e, "cudaGetDevice"); }
   e = configure_kernels(&h->max_smem);
   if (e != cudaSuccess) { delete h; return cuda_fail(e, "configure kernels"); }
-  h->st.setup(nfftx, nffty, nfftz, order);
+  h->st.setup(nfftx, nffty, nfftz, order, sm_count(h->device));
   apply_cached_config(h);
   const size_t bytes = SystemState::bytes(nfftx, nffty, nfftz);
   if (cudaMalloc(&h->d_block, bytes) != cudaSuccess ||
@@ -747,7 +744,7 @@ int pme_batch_create(const pme_system_desc* systems, int nsys, void* stream, pme
   std::vector<size_t> off(nsys), boff(nsys);
   size_t total = 0;
   for (int i = 0; i < nsys; i++) {
-    b->st[i].setup(systems[i].nfftx, systems[i].nffty, systems[i].nfftz, systems[i].order, false);
+    b->st[i].setup(systems[i].nfftx, systems[i].nffty, systems[i].nfftz, systems[i].order, 0);
     off[i] = total;
     total += SystemState::bytes(systems[i].nfftx, systems[i].nffty, systems[i].nfftz);
   }
@@ -841,7 +838,7 @@ int pme_batch_commit(pme_batch* b) {
   if (e == cudaSuccess) e = cudaMemcpy(b->d_prefix, prefix.data(), prefix.size() * sizeof(int), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cuda_fail(e, "batch: upload descriptors");
   b->smem = smem;
-  e = fused_shape(b->total, smem, b->grid_cap, false, &b->shape);
+  e = fused_shape(b->total, smem, b->grid_cap, 0, &b->shape);
   if (e != cudaSuccess) return cuda_fail(e, "batch: launch shape (does the kernel fit on an SM?)");
   return PME_OK;
 }

@@ -89,14 +89,9 @@ struct FusedShape {
   int cluster;   // > 0: launched with thread-block clusters of this many CTAs (latency build)
 };
 // Picks the build and the CTAs (at most the resident maximum, at most the largest phase's tile
-// count, at most grid_cap when > 0) for phases of total[] tiles and smem bytes per CTA; heavy: the
-// spread tiles are long (see heavy_tiles).
-cudaError_t fused_shape(const int* total, size_t smem, int grid_cap, bool heavy, FusedShape* out);
-// Whether a system's spread tiles take long beside the phases that only the latency build fuses: at
-// least 25,000 contributions each (about 20 us).
-inline bool heavy_tiles(const SysDesc& d) {
-  return (double)d.natom * d.order * d.order * d.order >= 25000.0 * tiles_blocks(d);
-}
+// count, at most grid_cap when > 0) for phases of total[] tiles and smem bytes per CTA; ctas: the CTAs
+// per SM that a single system's row blocks were chosen for (SystemState::ctas).
+cudaError_t fused_shape(const int* total, size_t smem, int grid_cap, int ctas, FusedShape* out);
 cudaError_t fused_launch(const FusedArgs& a, const FusedShape& shape, size_t smem, cudaStream_t s);
 // The same for a launch with clusters of cs CTAs (the cluster plane tiles).
 cudaError_t fused_shape_cluster(const int* total, size_t smem, int grid_cap, int cs, FusedShape* out);

@@ -485,21 +485,16 @@ static cudaError_t occupancy(size_t smem, Occupancy* out) {
   return cudaSuccess;
 }
 
-cudaError_t fused_shape(const int* total, size_t smem, int grid_cap, bool heavy, FusedShape* out) {
+cudaError_t fused_shape(const int* total, size_t smem, int grid_cap, int ctas, FusedShape* out) {
   Occupancy o;
   cudaError_t e = occupancy(smem, &o);
   if (e != cudaSuccess) return e;
   const int sms = o.sms, occ_lat = o.lat, occ_tput = o.tput;
   int most = 1;
   for (int p = 0; p < kPhases; p++) most = most > total[p] ? most : total[p];
-  // many tiles per CTA: more resident CTAs pay; about one: fewer registers per thread cost, unless
-  // the row blocks' tiles are long and 3 CTAs per SM take them in fewer waves (54,000 atoms,
-  // 90 x 75 x 80, order 8, 380 tiles: 188 us with 2 per SM, 167 with 3)
-  bool tput = occ_tput > occ_lat && most > 2 * sms * occ_lat;
-  if (!tput && heavy && occ_tput > occ_lat) {
-    const int wl = (total[1] + sms * occ_lat - 1) / (sms * occ_lat), wt = (total[1] + sms * occ_tput - 1) / (sms * occ_tput);
-    tput = 5 * wt < 4 * wl;   // a tile with 2 CTAs on its SM takes 0.8 of its time with 3
-  }
+  // a single system: the build that its row blocks were chosen for, where the third CTA fits; several:
+  // many tiles per CTA, more resident CTAs pay; about one, fewer registers per thread cost
+  const bool tput = occ_tput > occ_lat && (ctas > 0 ? ctas > 2 : most > 2 * sms * occ_lat);
   out->variant = tput ? kFusedThroughput : kFusedLatency;
   out->cluster = 0;
   int grid = sms * (tput ? occ_tput : occ_lat);

@@ -176,7 +176,7 @@ struct Request {
 
 size_t request_bytes(const pme_request& q) {
   SystemState st;
-  st.setup(q.nfftx, q.nffty, q.nfftz, q.order, false);
+  st.setup(q.nfftx, q.nffty, q.nfftz, q.order, 0);
   const int n = std::max(q.natom, 1);
   const size_t stride = (size_t)((n + 63) / 64) * 64;
   return align256(SystemState::bytes(q.nfftx, q.nffty, q.nfftz)) + align256(st.bin_ints(n) * sizeof(int)) +
@@ -323,7 +323,7 @@ void release_staging(pme_server* s, Request* q) {
 // Allocate, clear and fill the device state of a pending request (worker thread, lock held).
 int admit(pme_server* s, Request* q) {
   const pme_request& r = q->r;
-  q->st.setup(r.nfftx, r.nffty, r.nfftz, r.order, false);
+  q->st.setup(r.nfftx, r.nffty, r.nfftz, r.order, 0);
   const size_t sys = align256(SystemState::bytes(r.nfftx, r.nffty, r.nfftz));
   const size_t bins = align256(q->st.bin_ints(r.natom) * sizeof(int));
   const size_t xb = align256((size_t)r.natom * 16);
@@ -404,7 +404,7 @@ int rebuild(pme_server* s) {
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(s->d_slots, st + align256(tb) + align256(pb), sb, cudaMemcpyHostToDevice, s->stream);
   if (e != cudaSuccess) return cuda_fail(e, "server: upload tables");
-  e = fused_shape(s->total, s->smem, 0, false, &s->shape);
+  e = fused_shape(s->total, s->smem, 0, 0, &s->shape);
   if (e != cudaSuccess) return cuda_fail(e, "server: launch shape");
   return PME_OK;
 }

@@ -176,6 +176,8 @@ struct SystemState {
   FftPlan1D px{}, py{}, pz{};
   int tx_rows = 0, tx_y = 0, tx_z = 0, plane = 0;
   int bry = 4, brz = 4, nby = 1, nbz = 1;
+  int ctas = 0;              // CTAs per SM that the row blocks were chosen for: 2 the latency build, 3 the
+                             // throughput build (0: shared launches, whose tile counts decide)
   int bin_cap = 0, atom_cap = 0;
   int* bins = nullptr;       // counts, bin records, bookkeeping, overflow records, atom order
   unsigned long long* accum = nullptr;
@@ -197,8 +199,9 @@ struct SystemState {
            align256(4 * n * 8) + align256(kAccCount * 8) + align256(kEvCount * 8);
   }
 
-  // alone: the system has launches of its own (else it shares them with a batch or a server's requests)
-  void setup(int nx_, int ny_, int nz_, int order_, bool alone = true) {
+  // sms: the device's SM count, where the system has launches of its own; 0: it shares them with a batch
+  // or a server's requests
+  void setup(int nx_, int ny_, int nz_, int order_, int sms) {
     nx = nx_; ny = ny_; nz = nz_; order = order_;
     factorize(nx, px);
     factorize(ny, py);
@@ -211,54 +214,59 @@ struct SystemState {
     tx_z = pick_cols_tile(ny, nz);
     // whole-plane tiles need one thread per line of each orientation and the plane in smem
     plane = (plane_smem_bytes(ny, nz) <= kTileSmemBudget && ny <= kThreads && nz <= kThreads) ? 1 : 0;
-    pick_block(alone);
+    pick_block(sms);
+  }
+
+  // Row blocks of the fused spread + x pass (and of the gather), and the build of the kernel that runs
+  // them.  In launches with many systems, the largest square block that fits: fewest candidate records
+  // per contribution.  For a system alone, the block and CTAs per SM whose tiles take the least time in
+  // whole waves (block_cost).  The order can change later (pme_set_order): every block is one that fits
+  // at every order.
+  void pick_block(int sms) {
+    double best = 0.0;
+    bry = brz = 1;
+    ctas = sms > 0 ? 2 : 0;
+    for (int by = kSpreadMaxBlock; by >= 1; by--)
+      for (int bz = by; bz >= (sms > 0 ? 1 : by); bz--) {
+        size_t need = 0;
+        for (int o = 4; o <= kMaxOrder; o += 2) need = std::max(need, spread_x_smem_bytes(nx, by * bz, o));
+        if (need > kTileSmemBudget || (sms == 0 && best > 0.0)) continue;
+        for (int c = 2; c <= (sms > 0 ? 3 : 2); c++) {
+          const double cost = sms > 0 ? block_cost(by, bz, c, sms) : 1.0;
+          if (cost > 0.0 && (best == 0.0 || cost < best)) {
+            best = cost;
+            bry = by;
+            brz = bz;
+            ctas = sms > 0 ? c : 0;
+          }
+        }
+      }
     nby = (ny + bry - 1) / bry;
     nbz = (nz + brz - 1) / brz;
   }
 
-  // Row blocks of the fused spread + x pass (and of the gather).  In launches with many systems, the
-  // largest square block that fits: fewest candidate records per contribution.  For a system alone, the
-  // block whose tiles take the least time in whole waves of resident CTAs, by a model fitted to phase
-  // traces at 0.1 atoms per grid point: a tile takes 2.5 us + 10.2 ns per candidate record (of every bin
-  // its window touches) + 0.56 ns per contribution with 3 CTAs on an SM, 0.8 of that with 2; the build
-  // with 3 per SM runs more phases (8 us); a CTA more costs the barriers 6 ns; shared memory that leaves
-  // less L1 costs up to 15% (216^3, 68 against 56 KB a CTA: gather 284 and 270 us).  Spread phase, model
-  // and trace, us: 120 x 108 x 96 order 6, blocks of 4 x 4 rows 86 and 85, 4 x 3 66 and 71, 3 x 3 76 and 77;
-  // 90 x 75 x 80 order 8, 4 x 4 57 and 55, 3 x 3 78 and 76; 216^3 order 6, 3 x 3 (of 4 x 3 and 3 x 2) 482.
-  void pick_block(bool alone) {
-    double best = 0.0;
-    bool first = false;   // best is the largest block's
-    bry = brz = 1;
-    for (int by = kSpreadMaxBlock; by >= 1; by--)
-      for (int bz = by; bz >= (alone ? 1 : by); bz--) {
-        size_t need = 0;   // the order can change later (pme_set_order): size for every order
-        for (int o = 4; o <= kMaxOrder; o += 2) need = std::max(need, spread_x_smem_bytes(nx, by * bz, o));
-        if (need > kTileSmemBudget) continue;
-        if (!alone) {
-          bry = brz = by;
-          return;
-        }
-        const double tiles = (double)((ny + by - 1) / by) * ((nz + bz - 1) / bz), per_row = 0.1 * nx;
-        const double cand = by * ((order - 2 + by) / by + 1) * bz * ((order - 2 + bz) / bz + 1);   // rows of the bins
-        const double tile = 2.5 + per_row * (10.2e-3 * cand + 0.56e-3 * order * order * order * by * bz);
-        const size_t smem = spread_x_smem_bytes(nx, by * bz, order) + 2048;
-        double cost = 0.0;
-        for (int ctas = 2; ctas <= 3; ctas++) {   // latency build, throughput build
-          if (ctas * smem > 227 * 1024) continue;
-          const double l1 = 1.0 + 0.15 * (double)(ctas * smem) / (227 * 1024);
-          const double c = std::ceil(tiles / (148.0 * ctas)) * tile * l1 * (ctas == 2 ? 0.8 : 1.0) + (ctas == 2 ? 0.0 : 8.0) +
-                           6e-3 * std::min(tiles, 148.0 * ctas);
-          if (cost == 0.0 || c < cost) cost = c;
-        }
-        // the largest block, the first that fits, gives way to a clear gain only (128 x 125 x 128 order 4,
-        // predicted 0.98: 220 us with the smaller block, 216 without; 160^3, predicted 0.91: 318 and 348)
-        if (best == 0.0 || cost < (first ? 0.97 : 1.0) * best) {
-          first = best == 0.0;
-          best = cost;
-          bry = by;
-          brz = bz;
-        }
-      }
+  // Estimated cost of an evaluation's row-block tiles, by x bz rows each and c CTAs per SM; 0 where c do not
+  // fit.  A tile costs 6 + 18.5e-3 per candidate record (of every bin that its window touches) + 0.56e-3
+  // per contribution with 3 CTAs on its SM, less with fewer beside it: 0.76 to 0.78 of that with 2 (0.70 at
+  // order 8), 0.55 alone; 6% more where the SM's shared memory grows beyond 196 KB, to its largest size,
+  // and leaves the gather less L1.  Fitted to whole evaluations of 267 systems (18^3 to 216^3, uneven ones
+  // among them, orders 4, 6 and 8, 0.1 to 0.144 atoms per grid point, 9 to 12 pairs of block and build
+  // each): the pair chosen takes 0.4% more than the best one measured on average, 12% at most (96^3 order
+  // 6, 168 and 150 us).  72^3 order 4: 3 x 3 rows with 2 CTAs 86 us, with 3 82, 4 x 4 rows with 3 75;
+  // 144^3 order 4, 4 x 3 rows: 300 us with 2, 266 with 3; 150^3 order 8, 4 x 4 rows: 613 and 719.
+  double block_cost(int by, int bz, int c, int sms) const {
+    SysDesc d = desc(nullptr, 0.0, nullptr, 0, nullptr, 0, 0, 0, 0);
+    d.plane = 0;
+    d.bry = by;
+    d.brz = bz;
+    const size_t smem = c * (fused_smem_bytes(d) + 2064);   // the kernels' static part, what each CTA reserves
+    if (smem > 228 * 1024) return 0.0;
+    const double tiles = (double)((ny + by - 1) / by) * ((nz + bz - 1) / bz), per_row = 0.1 * nx;
+    const double cand = by * ((order - 2 + by) / by + 1) * bz * ((order - 2 + bz) / bz + 1);   // rows of the bins
+    const double tile = 6.0 + per_row * (18.5e-3 * cand + 0.56e-3 * order * order * order * by * bz);
+    const double two = order == 4 ? 0.78 : (order == 6 ? 0.76 : 0.70);
+    const double share = c == 3 ? 1.0 : (tiles <= sms ? 0.55 : two);
+    return std::ceil(tiles / (c * sms)) * tile * share * (smem > 196 * 1024 ? 1.06 : 1.0) + (c == 3 ? 1.0 : 0.0);
   }
 
   int nbins() const { return nby * nbz; }

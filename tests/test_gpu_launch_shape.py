@@ -1,0 +1,61 @@
+"""The launch of a single system's evaluation: the build of the kernel is the one that the row blocks were
+chosen for, and the inverse x pass runs inside the gather only where the gather is one wave.  The shapes
+change the time alone: forces, energy and virial are the staged calls', bit for bit."""
+import numpy as np
+import pytest
+
+from gpu_recip_b200 import systems as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(nfft, order):
+    box = tuple(float(n) for n in nfft)
+    waters = int(np.prod(box) * 8000 / 62.1 ** 3)
+    return S.PmeSystem("launch", S.water_box(waters, box, 5), box, nfft, order, 0.33)
+
+
+def _eval(torch, p, s, x, staged=False):
+    from gpu_recip_b200 import recip_from_box
+    f = torch.zeros((s.natom, 3), device="cuda")
+    r = recip_from_box(s.box)
+    p.energy_virial.clear()
+    if staged:
+        p.spread_charge(x, s.natom, r)
+        p.r2c_fft()
+        p.scalar_sum(r, s.kappa, True, True)
+        p.c2r_fft()
+        p.gather_force(x, s.natom, r, 1, f)
+    else:
+        p.eval(r, x, s.natom, s.kappa, True, True, f, 1)
+    p.energy_virial.copyToHost()
+    return f.cpu().numpy(), p.energy_virial.getEnergy("recip"), p.energy_virial.getVirial()
+
+
+@pytest.mark.parametrize("nfft,order,three,fused_x", [
+    ((64, 64, 64), 4, False, True),       # 256 tiles of 4 x 4 rows: one wave of 2 CTAs per SM
+    ((40, 128, 64), 4, False, False),     # 512: more than one wave
+    ((72, 72, 72), 4, True, False),       # 432 of 4 x 3 rows: one wave of 3 CTAs per SM
+    ((81, 81, 81), 6, True, False),       # 441 of 4 x 4 rows
+    ((90, 75, 80), 8, True, False),       # 380 of 4 x 4 rows
+    ((128, 125, 128), 8, False, False),   # 1024 of 4 x 4 rows: faster in four waves of 2 than in three of 3
+])
+def test_build_follows_the_row_blocks(cuda, nfft, order, three, fused_x):
+    from gpu_recip_b200 import CudaPMERecip
+    from gpu_recip_b200.pme import TRACE_STEP_STAMPS
+    sms = cuda.cuda.get_device_properties(0).multi_processor_count
+    if sms != 148:
+        pytest.skip("the tile counts are for 148 SMs")
+    s = _system(nfft, order)
+    x = cuda.from_numpy(s.xyzq).cuda()
+    p = CudaPMERecip(*nfft, order)
+    buf = cuda.zeros(1024 * 14 + TRACE_STEP_STAMPS, dtype=cuda.int64, device="cuda")
+    p.set_trace(buf, 1024)
+    got = _eval(cuda, p, s, x)
+    p.set_trace(None)
+    ran = buf[:1024 * 14].view(1024, 7, 2)[:, :, 0].cpu().numpy() > 0
+    assert (ran[:, 1].sum() > 2 * sms) == three
+    assert ran[:, 5].any() != fused_x
+    want = _eval(cuda, CudaPMERecip(*nfft, order), s, x, staged=True)
+    assert np.array_equal(got[0], want[0]) and got[1] == want[1] and np.array_equal(got[2], want[2])
+    p.close()
