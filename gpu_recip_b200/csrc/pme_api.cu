@@ -328,6 +328,10 @@ int pme_set_order(pme_recip* h, int order) {
   cudaError_t e = cudaStreamSynchronize(h->stream);   // tables are replaced synchronously
   if (e != cudaSuccess) return cuda_fail(e, "set_order");
   h->st.order = order;
+  // without bins yet, the new order's own row block; else the block in place keeps its storage (a captured
+  // evaluation may hold it) and only the build follows the order
+  if (h->d_bins) h->st.pick_build(sm_count(h->device));
+  else h->st.pick_block(sm_count(h->device));
   e = h->st.upload_tables();
   if (e != cudaSuccess) return cuda_fail(e, "set_order: upload moduli");
   return PME_OK;

@@ -245,6 +245,12 @@ struct SystemState {
     nbz = (nz + brz - 1) / brz;
   }
 
+  // The build for the block in place (after a change of the order).
+  void pick_build(int sms) {
+    const double three = block_cost(bry, brz, 3, sms);
+    ctas = three > 0.0 && three < block_cost(bry, brz, 2, sms) ? 3 : 2;
+  }
+
   // Estimated cost of an evaluation's row-block tiles, by x bz rows each and c CTAs per SM; 0 where c do not
   // fit.  A tile costs 6 + 18.5e-3 per candidate record (of every bin that its window touches) + 0.56e-3
   // per contribution with 3 CTAs on its SM, less with fewer beside it: 0.76 to 0.78 of that with 2 (0.70 at

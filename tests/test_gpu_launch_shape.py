@@ -1,6 +1,8 @@
 """The launch of a single system's evaluation: the build of the kernel is the one that the row blocks were
 chosen for, and the inverse x pass runs inside the gather only where the gather is one wave.  The shapes
 change the time alone: forces, energy and virial are the staged calls', bit for bit."""
+import functools
+
 import numpy as np
 import pytest
 
@@ -9,6 +11,7 @@ from gpu_recip_b200 import systems as S
 pytestmark = pytest.mark.gpu
 
 
+@functools.lru_cache(maxsize=None)
 def _system(nfft, order):
     box = tuple(float(n) for n in nfft)
     waters = int(np.prod(box) * 8000 / 62.1 ** 3)
@@ -58,4 +61,43 @@ def test_build_follows_the_row_blocks(cuda, nfft, order, three, fused_x):
     assert ran[:, 5].any() != fused_x
     want = _eval(cuda, CudaPMERecip(*nfft, order), s, x, staged=True)
     assert np.array_equal(got[0], want[0]) and got[1] == want[1] and np.array_equal(got[2], want[2])
+    p.close()
+
+
+def test_changed_order_takes_its_own_row_block(cuda):
+    """Order 8 on 32^3 has blocks of 4 x 1 rows (256 tiles), order 4 of 3 x 3 (121): a handle whose order
+    changes before its first evaluation is launched as one made with that order."""
+    from gpu_recip_b200 import CudaPMERecip
+    from gpu_recip_b200.pme import TRACE_STEP_STAMPS
+    s = _system((32, 32, 32), 4)
+    x = cuda.from_numpy(s.xyzq).cuda()
+    tiles = []
+    for first in (4, 8):
+        p = CudaPMERecip(32, 32, 32, first)
+        p.set_order(4)
+        buf = cuda.zeros(1024 * 14 + TRACE_STEP_STAMPS, dtype=cuda.int64, device="cuda")
+        p.set_trace(buf, 1024)
+        _eval(cuda, p, s, x)
+        p.set_trace(None)
+        tiles.append(int((buf[:1024 * 14].view(1024, 7, 2)[:, 1, 0] > 0).sum()))
+        p.close()
+    assert tiles[0] == tiles[1]
+
+
+@pytest.mark.parametrize("evaluated", [False, True])
+@pytest.mark.parametrize("nfft", [(32, 32, 32), (72, 72, 72)])
+@pytest.mark.parametrize("first,order", [(4, 8), (8, 4), (6, 4), (4, 6)])
+def test_changed_order_gives_a_new_handles_bits(cuda, nfft, first, order, evaluated):
+    """Whether or not the handle has evaluated at its first order: order 4 to 8 and back."""
+    from gpu_recip_b200 import CudaPMERecip
+    s = _system(nfft, order)
+    x = cuda.from_numpy(s.xyzq).cuda()
+    p = CudaPMERecip(*nfft, first)
+    if evaluated:
+        _eval(cuda, p, s, x)
+    p.set_order(order)
+    want = _eval(cuda, CudaPMERecip(*nfft, order), s, x)
+    for _ in range(2):
+        got = _eval(cuda, p, s, x)
+        assert np.array_equal(got[0], want[0]) and got[1] == want[1] and np.array_equal(got[2], want[2])
     p.close()
