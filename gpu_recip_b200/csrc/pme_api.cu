@@ -83,6 +83,7 @@ struct pme_batch {
   int grid_cap = 0;
   int line_scale = 0;   // lines per x/y/z pass tile: each system's default times this (budget permitting);
                         // 0: the largest of 4, 2 and 1 that leaves the launch two waves of x-pass tiles
+  int laid_scale = 1;   // the multiplier that the present tiles were laid out with
 };
 
 namespace {
@@ -826,6 +827,7 @@ int pme_batch_commit(pme_batch* b) {
   };
   if (b->line_scale > 0) {
     smem = lay_out(b->line_scale, kTileSmemBudget);
+    b->laid_scale = b->line_scale;
   } else {
     // a 16-line tile of a short length is mostly its own latency (256 systems: 1,618 us at 1,
     // 1,496 at 4, the x inverse 275 and 152);
@@ -833,6 +835,7 @@ int pme_batch_commit(pme_batch* b) {
     const size_t budget = lay_out(1, kTileSmemBudget) - 2048;   // less what a tile needs beside its lines
     for (int scale : {4, 2, 1}) {
       smem = lay_out(scale, scale == 1 ? kTileSmemBudget : budget);
+      b->laid_scale = scale;
       if (prefix[(size_t)5 * (nsys + 1) + nsys] >= 2 * 3 * sm_count(b->device)) break;
     }
   }
@@ -1101,14 +1104,17 @@ int pme_batch_autotune(pme_batch* b, int reps, pme_tune_config* out) {
   const int sms = sm_count(b->device);
   const int start_mode = b->plane_mode, start_cap = b->grid_cap, start_scale = b->line_scale;
   int best_mode = start_mode, best_cap = start_cap, best_scale = start_scale, count = 0, rc = PME_OK;
+  int best_laid = 1, default_laid = 0;
   float best_us = 0.0f;
-  for (int scale : {1, 2, 4}) {
+  for (int scale : {0, 1, 2, 4}) {   // the untuned layout first: the others have to beat it
+    if (scale == 1 && default_laid == 1) continue;   // the same layout
     for (int mode : {PME_SCHED_AUTO, PME_SCHED_PASSES}) {
       for (int cap : {0, sms}) {
         b->plane_mode = mode;
         b->grid_cap = cap;
         b->line_scale = scale;
         if ((rc = pme_batch_commit(b))) break;
+        if (scale == 0) default_laid = std::max(default_laid, b->laid_scale);
         float us = 0.0f;
         rc = time_launches([&]() { return pme_batch_eval(b); }, b->stream, b->d_status, reps, ev, &us);
         if (rc) break;
@@ -1117,6 +1123,7 @@ int pme_batch_autotune(pme_batch* b, int reps, pme_tune_config* out) {
           best_mode = mode;
           best_cap = cap;
           best_scale = scale;
+          best_laid = b->laid_scale;
         }
         count++;
       }
@@ -1137,7 +1144,7 @@ int pme_batch_autotune(pme_batch* b, int reps, pme_tune_config* out) {
     std::memset(out, 0, sizeof(*out));
     out->schedule = best_mode;
     out->grid_ctas = best_cap;
-    out->x_lines = out->y_lines = out->z_columns = best_scale;   // multiplier of each system's default
+    out->x_lines = out->y_lines = out->z_columns = best_laid;   // multiplier of each system's default
     out->us_per_eval = best_us;
     out->candidates = count;
   }

@@ -141,3 +141,22 @@ def test_x_gather_fusion_rejects_unknown_modes(cuda):
     with pytest.raises(C.PMEError) as e:
         pme.set_x_gather_fusion(7)
     assert e.value.status == C.PME_EINVAL
+
+
+def test_batch_autotune_tries_the_untuned_layout(cuda):
+    """A batch whose untuned layout is none of the three multipliers' (tiles of up to 64 lines in the shared
+    memory that the launch takes anyway) measures it too, and keeps its results."""
+    torch = cuda
+    from gpu_recip_b200 import PmeBatch
+    specs, forces = [], []
+    for sy in S.batch_systems(96, seed=10):
+        forces.append(torch.zeros((sy.natom, 3), device="cuda"))
+        specs.append(dict(nfft=sy.nfft, order=sy.order, box=sy.box, kappa=sy.kappa,
+                          xyzq=torch.from_numpy(sy.xyzq).cuda(), force=forces[-1], stride=1))
+    b = PmeBatch(specs)
+    b.eval()
+    before = [f.clone() for f in forces]
+    cfg = b.autotune(reps=2)
+    assert cfg["candidates"] == 16 and cfg["x_lines"] in (1, 2, 4)
+    b.eval()
+    assert all(torch.equal(f, g) for f, g in zip(before, forces))
