@@ -43,8 +43,9 @@ constexpr int kSquareTypes = 64;      // vdW types up to which every CTA holds t
 constexpr int kMaxTypes = 200;        // vdW types
 constexpr float kEnergyScale = 4294967296.0f;     // 2^32
 constexpr float kForceScaleF = 1099511627776.0f;  // 2^40
+constexpr int kTabShift = 15;        // high word of r^2 -> table interval
+static_assert(kTabOctave == 1 << (20 - kTabShift), "the interval's bits");
 constexpr float kTwoSqrtPi = 1.1283791670955126f; // 2/sqrt(pi)
-constexpr int kTabOctave = 64, kTabMax = 16 * kTabOctave;   // Ewald table intervals (see ensure_ewald)
 
 struct Params {
   float box[3], inv_box[3];
@@ -60,9 +61,8 @@ struct Params {
   int slices;         // tasks per cluster, each with some of the column rows along z
   double kappad, roff2d, ro6d, ro12d, ro18d;   // FP64 for the main-list pair terms
   double boxd[3];
-  // Ewald real space, cubics on the intervals of s = r^2 that share their leading float bits (kTabOctave
-  // per factor of two, from s = 2): F = (r dE/dr) / r^2 of E = erfc(kappa r) / r, then E itself
-  const double4* tab;
+  // Ewald real space (ewald_table): F = (r dE/dr) / r^2 of E = erfc(kappa r) / r, then E itself
+  const double2* tab;
   int tab_n;          // intervals (0: no table); s outside them uses erfc() and exp()
 };
 
@@ -108,9 +108,10 @@ __device__ __forceinline__ double reciprocal(double x) {
   return __fma_rn(y, __fma_rn(e, e, e), y);
 }
 
-__device__ __forceinline__ double cubic(const double2* c, double t) {
-  const double2 lo = c[0], hi = c[1];
-  return __fma_rn(__fma_rn(__fma_rn(hi.y, t, hi.x), t, lo.y), t, lo.x);
+static_assert(kTabTerms == 6, "quintics");
+__device__ __forceinline__ double quintic(const double2* c, double t) {
+  const double2 lo = c[0], mid = c[1], hi = c[2];
+  return __fma_rn(__fma_rn(__fma_rn(__fma_rn(__fma_rn(hi.y, t, hi.x), t, mid.y), t, mid.x), t, lo.y), t, lo.x);
 }
 
 // Shifted Lennard-Jones: (r dU/dr) and U from s = r^2 and 1 / s.
@@ -310,11 +311,11 @@ __global__ void __launch_bounds__(kWarps * 32, kPairCtas) k_direct_pairs(
     const ulonglong2* __restrict__ mask, const int* __restrict__ far_ptr, const int* __restrict__ far_idx,
     const float2* __restrict__ vdwp, int calc_energy, int calc_virial, int stride, long long* __restrict__ force,
     long long* __restrict__ acc, int* __restrict__ next_task) {
-  extern __shared__ double2 sh_dyn[];   // Ewald cubics (with EV: F and E of an interval together), then vdW table
-  constexpr int kEntry = EV ? 4 : 2;    // double2 per interval
+  extern __shared__ double2 sh_dyn[];   // Ewald quintics (with EV: F and E of an interval together), then vdW table
+  constexpr int kEntry = EV ? 6 : 3;    // double2 per interval
   float2* const sh_vdw = reinterpret_cast<float2*>(sh_dyn + kEntry * p.tab_n);
   for (int k = threadIdx.x; k < kEntry * p.tab_n; k += blockDim.x)
-    sh_dyn[k] = __ldg(reinterpret_cast<const double2*>(p.tab) + (EV ? k : (k >> 1) * 4 + (k & 1)));
+    sh_dyn[k] = __ldg(p.tab + (EV ? k : k + k / 3 * 3));
   __shared__ int2 sh_queue[kWarps][kCluster][kQueue + 1];   // j and its image (2 bits per axis)
   __shared__ ulonglong2 sh_xy[kWarps][kCluster / 2];        // the cluster's coordinates, atoms in pairs
   __shared__ unsigned long long sh_z[kWarps][kCluster / 2];
@@ -499,12 +500,12 @@ __global__ void __launch_bounds__(kWarps * 32, kPairCtas) k_direct_pairs(
         bool slow = false;
         // Ewald: the interval is the exponent and leading bits of r^2, t its offset from the middle
         const int hi_s = __double2hiint(r2);
-        const unsigned at_s = (unsigned)(hi_s >> 14) - (0x40000000u >> 14);
+        const unsigned at_s = (unsigned)(hi_s >> kTabShift) - (0x40000000u >> kTabShift);
         if (STD || p.tab_n > 0) {
-          const double t = r2 - __hiloint2double((hi_s & ~0x3fff) | 0x2000, 0);
+          const double t = r2 - __hiloint2double((hi_s & -(1 << kTabShift)) | 1 << (kTabShift - 1), 0);
           const double2* const c = sh_dyn + kEntry * (at_s < (unsigned)p.tab_n ? at_s : 0u);
-          f = qq * cubic(c, t);
-          if (EV) ue = qq * cubic(c + 2, t);
+          f = qq * quintic(c, t);
+          if (EV) ue = qq * quintic(c + 3, t);
         }
         if (STD || p.elec != PME_ELEC_NONE) slow = at_s >= (unsigned)p.tab_n;
         if (STD || vdw_on) {
@@ -676,7 +677,7 @@ struct pme_direct {
   int* d_far_ptr = nullptr;
   int* d_far_idx = nullptr;
   bool excl_set = false;
-  double4* d_tab = nullptr;  // Ewald table for the current kappa and roff (see ensure_ewald)
+  double* d_tab = nullptr;   // Ewald table for the current kappa and roff
   int tab_n = 0;
   double tab_kappa = -1.0, tab_roff = -1.0;
   int4* d_list14 = nullptr;
@@ -744,51 +745,23 @@ Params make_params(const pme_direct* h) {
   const double longest = std::max(h->box[0], std::max(h->box[1], h->box[2]));
   p.cut2 = p.roff2 * 1.00001f + (float)(1e-6 * longest * h->roff);
   p.marg = (float)(1e-5 + 1e-6 * longest);
-  p.tab = h->d_tab;
+  p.tab = reinterpret_cast<const double2*>(h->d_tab);
   p.tab_n = h->elec_model == PME_ELEC_NONE ? 0 : h->tab_n;
   return p;
 }
 
-// Cubic through f at the four Chebyshev points of [mid - half, mid + half], as coefficients of 1, t,
-// t^2, t^3, t = s - mid (Newton's divided differences, expanded).
-template <class F>
-double4 chebyshev_cubic(F f, double mid, double half) {
-  double x[4], d[4];
-  for (int i = 0; i < 4; i++) {
-    x[i] = half * std::cos(kPi * (2 * i + 1) / 8.0);
-    d[i] = f(mid + x[i]);
-  }
-  for (int k = 1; k < 4; k++)
-    for (int i = 3; i >= k; i--) d[i] = (d[i] - d[i - 1]) / (x[i] - x[i - k]);
-  return make_double4(d[0] - x[0] * (d[1] - x[1] * (d[2] - x[2] * d[3])),
-                      d[1] - (x[0] + x[1]) * d[2] + (x[0] * x[1] + x[0] * x[2] + x[1] * x[2]) * d[3],
-                      d[2] - (x[0] + x[1] + x[2]) * d[3], d[3]);
-}
-
-// Table of F(s) = (r dE/dr) / s and E(s) = erfc(kappa r) / r, s = r^2, from s = 2 to roff^2 (close
-// pairs use the formulas): two cubics per interval, kTabOctave intervals per factor of two, so that
-// the interval is read off the float's leading bits.  Largest errors for r >= 1.5 A: 6e-11 of E, 3e-10
-// of F r (a cubic Hermite table of 4,096 even intervals, gathered from global memory, had 6e-11 and
-// 4e-10).  11 KB of F for roff = 9 A sit in every CTA's shared memory: two 16-byte loads and three
-// FMAs per pair, against 26 coefficients fetched and 37 FP64 operations for polynomials over the whole
-// range (192,000 atoms: 784 against 945 us).
+// The Ewald table in device memory (close pairs, s < 2, use the formulas).  Every CTA copies it to its
+// shared memory: 8 KB of F for roff = 9 A, 16 KB with E; three 16-byte loads and five FMAs per pair.
+// 192,000 atoms, forces only, 730 us, error against 64 bits 6.9e-10; cubics on twice the intervals 722 us and
+// 1.9e-9; polynomials over the whole range (26 coefficients fetched and 37 FP64 operations) a fifth slower.
 int ensure_ewald(pme_direct* h) {
   if (h->elec_model == PME_ELEC_NONE) return PME_OK;
   if (h->tab_kappa == h->kappa && h->tab_roff == h->roff) return PME_OK;
   h->tab_kappa = -1.0;
-  const double k = h->kappa, c1 = 2.0 / std::sqrt(kPi) * k, s1 = h->roff * h->roff;
-  std::vector<double4> t;
-  for (int i = 0; i < kTabMax; i++) {
-    const double w = std::ldexp(2.0, i / kTabOctave) / kTabOctave, a = (kTabOctave + i % kTabOctave) * w;
-    if (a > s1) break;
-    auto E = [&](double s) { const double r = std::sqrt(s); return std::erfc(k * r) / r; };
-    auto F = [&](double s) { return (-c1 * std::exp(-k * k * s) - E(s)) / s; };
-    t.push_back(chebyshev_cubic(F, a + 0.5 * w, 0.5 * w));
-    t.push_back(chebyshev_cubic(E, a + 0.5 * w, 0.5 * w));
-  }
+  const std::vector<double> t = ewald_table(h->kappa, h->roff);
   cudaError_t e = upload(&h->d_tab, t.data(), t.size(), h->stream);
   if (e != cudaSuccess) return cuda_fail(e, "direct: Ewald table");
-  h->tab_n = (int)(t.size() / 2);
+  h->tab_n = (int)(t.size() / (2 * kTabTerms));
   h->tab_kappa = h->kappa;
   h->tab_roff = h->roff;
   return PME_OK;
@@ -1098,7 +1071,7 @@ int pme_direct_calc_force(pme_direct* h, const void* xyzq, int ncoord, int calc_
   const bool std_terms = h->vdw_model != PME_VDW_NONE && p.square && p.tab_n > 0;
   auto kern = std_terms ? (ev ? k_direct_pairs<true, true> : k_direct_pairs<false, true>)
                         : (ev ? k_direct_pairs<true, false> : k_direct_pairs<false, false>);
-  const size_t smem = (size_t)p.tab_n * (ev ? 2 : 1) * sizeof(double4) +
+  const size_t smem = (size_t)p.tab_n * (ev ? 2 : 1) * kTabTerms * sizeof(double) +
                       (size_t)(p.square ? p.ntype * p.ntype : 0) * sizeof(float2);
   // one wave of resident CTAs; their warps draw the tasks from a counter.  Few clusters: more tasks
   // each, so that the last ones to finish are short

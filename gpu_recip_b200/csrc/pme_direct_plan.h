@@ -1,10 +1,12 @@
-// pme_direct_plan.h -- host-side choices of the direct-space engine that need no device: the columns and
-// x bins that the atoms are sorted into.  Plain C++, so that they can be checked without a GPU.
+// pme_direct_plan.h -- host-side choices and tables of the direct-space engine that need no device: the
+// columns and x bins that the atoms are sorted into, the Ewald table.  Plain C++, so that they can be
+// checked without a GPU.
 #pragma once
 
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
+#include <vector>
 
 namespace pme {
 namespace direct {
@@ -54,6 +56,55 @@ inline int most_clusters(int n, const Columns& c) { return n / kCluster + std::m
 inline Columns room_columns(const double* box, double roff, int natom) {
   const double f = 1.05, b[3] = {f * box[0], f * box[1], f * box[2]};
   return plan_columns(b, roff, (int)std::min(2147483647.0, std::ceil(f * f * f * natom)));
+}
+
+// Ewald table: polynomials on the intervals of s = r^2 that share their leading float bits, kTabOctave
+// per factor of two from s = 2 on, so that the interval is read off the bits.
+constexpr int kTabOctave = 32, kTabTerms = 6, kTabMax = 16 * kTabOctave;
+
+// Polynomial through f at the kTabTerms Chebyshev points of [mid - half, mid + half]: coefficients of
+// 1, t, t^2, ..., t = s - mid (the Chebyshev series, written out in powers of t / half).
+template <class F>
+void chebyshev_powers(F f, double mid, double half, double* out) {
+  const double pi = 3.14159265358979323846;
+  double c[kTabTerms], prev[kTabTerms] = {1.0}, cur[kTabTerms] = {0.0, 1.0}, y[kTabTerms];
+  for (int k = 0; k < kTabTerms; k++) y[k] = f(mid + half * std::cos(pi * (k + 0.5) / kTabTerms));
+  for (int j = 0; j < kTabTerms; j++) {
+    c[j] = 0.0;
+    for (int k = 0; k < kTabTerms; k++) c[j] += (j == 0 ? 1.0 : 2.0) / kTabTerms * y[k] * std::cos(pi * j * (k + 0.5) / kTabTerms);
+  }
+  for (int i = 0; i < kTabTerms; i++) out[i] = c[0] * prev[i] + c[1] * cur[i];
+  for (int j = 2; j < kTabTerms; j++) {   // T_j = 2 z T_{j-1} - T_{j-2}
+    double next[kTabTerms];
+    for (int i = 0; i < kTabTerms; i++) next[i] = (i > 0 ? 2.0 * cur[i - 1] : 0.0) - prev[i];
+    for (int i = 0; i < kTabTerms; i++) {
+      out[i] += c[j] * next[i];
+      prev[i] = cur[i];
+      cur[i] = next[i];
+    }
+  }
+  double scale = 1.0;
+  for (int i = 0; i < kTabTerms; i++, scale /= half) out[i] *= scale;
+}
+
+// Per interval from s = 2 to roff^2 the coefficients of F(s) = (r dE/dr) / s, then of E(s) = erfc(kappa r)
+// / r.  Largest errors for r >= 1.5 A, kappa 0.32, cutoffs of 9 and 12 A: 3e-13 of F r, 5e-14 of E; rms over
+// the pairs 1.4e-14 and 4e-15.  (Cubics on 64 intervals per factor of two, a third larger: 3e-10 and
+// 6e-11, rms 1.5e-11 and 5e-12.  A cubic Hermite table of 4,096 even intervals, too large for shared
+// memory: 4e-10 and 6e-11 at 9 A, rms 6e-12 and 1e-12.)
+inline std::vector<double> ewald_table(double kappa, double roff) {
+  const double c1 = 2.0 / std::sqrt(3.14159265358979323846) * kappa;
+  auto E = [&](double s) { const double r = std::sqrt(s); return std::erfc(kappa * r) / r; };
+  auto F = [&](double s) { return (-c1 * std::exp(-kappa * kappa * s) - E(s)) / s; };
+  std::vector<double> t;
+  for (int i = 0; i < kTabMax; i++) {
+    const double w = std::ldexp(2.0, i / kTabOctave) / kTabOctave, a = (kTabOctave + i % kTabOctave) * w;
+    if (a > roff * roff) break;
+    t.resize(t.size() + 2 * kTabTerms);
+    chebyshev_powers(F, a + 0.5 * w, 0.5 * w, t.data() + t.size() - 2 * kTabTerms);
+    chebyshev_powers(E, a + 0.5 * w, 0.5 * w, t.data() + t.size() - kTabTerms);
+  }
+  return t;
 }
 
 }  // namespace direct

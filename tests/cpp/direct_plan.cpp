@@ -1,4 +1,4 @@
-// Host-side choices and sums of the direct-space engine, printed for tests/test_direct_plan.py (no GPU).
+// Host-side choices, tables and sums of the direct-space engine, printed for tests/test_direct_plan.py (no GPU).
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -38,8 +38,19 @@ static int sums() {
   return 0;
 }
 
+// kappa and cutoff per line of stdin -> the Ewald table, an interval's coefficients per line
+static int ewald() {
+  double kappa, roff;
+  while (std::scanf("%lf %lf", &kappa, &roff) == 2) {
+    const std::vector<double> t = ewald_table(kappa, roff);
+    for (size_t i = 0; i < t.size(); i++) std::printf(i % (2 * kTabTerms) == 2 * kTabTerms - 1 ? "%.17g\n" : "%.17g ", t[i]);
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   if (argc == 2 && !std::strcmp(argv[1], "columns")) return columns();
   if (argc == 2 && !std::strcmp(argv[1], "sums")) return sums();
+  if (argc == 2 && !std::strcmp(argv[1], "ewald")) return ewald();
   return 1;
 }
