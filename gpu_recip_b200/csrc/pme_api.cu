@@ -112,22 +112,25 @@ int ensure_bins(pme_recip* h, int natom) {
   SystemState& s = h->st;
   if (h->d_bins && natom <= s.atom_cap) return PME_OK;
   const int cap = std::max(natom, 1024);
-  const size_t ints = s.bin_ints(cap);
   cudaError_t e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return cuda_fail(e, "bins: sync");
   cudaFree(h->d_bins);
   h->d_bins = nullptr;
-  if (cudaMalloc(&h->d_bins, ints * sizeof(int)) != cudaSuccess) {
+  s.bin_cap = s.roomy_cap(cap);
+  if (cudaMalloc(&h->d_bins, s.bin_ints(cap, s.bin_cap) * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
-    s.bins = nullptr;
-    s.atom_cap = 0;
-    return fail(PME_ENOMEM, "device allocation of the atom bins failed");
+    s.bin_cap = SystemState::cap_for(cap, s.nbins());   // little memory left: what the results need
+    if (cudaMalloc(&h->d_bins, s.bin_ints(cap, s.bin_cap) * sizeof(int)) != cudaSuccess) {
+      cudaGetLastError();
+      s.bins = nullptr;
+      s.atom_cap = 0;
+      return fail(PME_ENOMEM, "device allocation of the atom bins failed");
+    }
   }
-  e = cudaMemset(h->d_bins, 0, ints * sizeof(int));
+  e = cudaMemset(h->d_bins, 0, s.bin_ints(cap, s.bin_cap) * sizeof(int));
   if (e != cudaSuccess) return cuda_fail(e, "bins: clear");
   s.bins = h->d_bins;
   s.atom_cap = cap;
-  s.bin_cap = SystemState::cap_for(cap, s.nbins());
   return PME_OK;
 }
 
@@ -643,7 +646,7 @@ int pme_get_status(pme_recip* h, int* device_status) {
     if (e == cudaSuccess) e = cudaMemsetAsync(h->st.accum, 0, h->st.G() * 8, h->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(h->st.acc, 0, kAccCount * sizeof(long long), h->stream);
     if (e == cudaSuccess && h->d_bins)
-      e = cudaMemsetAsync(h->d_bins, 0, h->st.bin_ints(h->st.atom_cap) * sizeof(int), h->stream);
+      e = cudaMemsetAsync(h->d_bins, 0, h->st.bin_ints(h->st.atom_cap, h->st.bin_cap) * sizeof(int), h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return cuda_fail(e, "get_status: reset");
     h->accum_zero = true;

@@ -277,16 +277,23 @@ struct SystemState {
 
   int nbins() const { return nby * nbz; }
 
-  // bin storage for up to natom atoms: capacity 1.5x the mean occupancy + 32 per bin
+  // Bin storage for up to natom atoms.  Atoms beyond a bin's capacity go to one list that every tile reads.
+  // Systems that share launches: capacity 1.5x the mean occupancy + 32 per bin.
   static int cap_for(int natom, int nbins) { return std::max(32, (int)(1.5 * natom / nbins) + 32); }
+  // A system alone: at least a bin full of liquid (0.2 atoms per grid point, at most 8x the mean), so that
+  // slabs and droplets in vacuum keep off that list too (144^3, 75,000 atoms in a quarter of the box, order 4
+  // 2,340 and 198 us, order 6 3,090 and 232, order 8 3,810 and 298).  At most 26 bytes per grid point.
+  int roomy_cap(int natom) const {
+    return std::max(cap_for(natom, nbins()), (int)std::min(8.0 * natom / nbins(), 0.2 * nx * bry * brz) + 32);
+  }
   // counts (padded to 16 bytes), bin records, bookkeeping (kMetaInts), overflow records, the
   // bin-sorted atom order; records are sized for order 8
   size_t count_ints() const { return (2 * (size_t)nbins() + 3) & ~(size_t)3; }
-  size_t bin_ints(int natom) const {
+  size_t bin_ints(int natom, int cap) const {
     const size_t n = (size_t)std::max(natom, 1);
-    return count_ints() + (size_t)nbins() * cap_for(natom, nbins()) * rec_floats(kMaxOrder) + kMetaInts +
-           n * rec_floats(kMaxOrder) + n;
+    return count_ints() + (size_t)nbins() * cap * rec_floats(kMaxOrder) + kMetaInts + n * rec_floats(kMaxOrder) + n;
   }
+  size_t bin_ints(int natom) const { return bin_ints(natom, cap_for(natom, nbins())); }
 
   void carve(char* base) {
     const size_t n = nx + ny + nz;
