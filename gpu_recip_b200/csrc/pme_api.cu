@@ -107,6 +107,12 @@ StagedCtx staged_ctx(const pme_recip* h) { return StagedCtx{h->d_bar, h->d_statu
 
 unsigned int* self_counter(const pme_recip* h) { return (unsigned int*)(h->d_bar + 4); }
 
+int sm_count(int dev) {
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 1;
+  return sms;
+}
+
 // Size the fused path's atom bins for natom atoms (allocates only when the count grows).
 int ensure_bins(pme_recip* h, int natom) {
   SystemState& s = h->st;
@@ -116,6 +122,10 @@ int ensure_bins(pme_recip* h, int natom) {
   if (e != cudaSuccess) return cuda_fail(e, "bins: sync");
   cudaFree(h->d_bins);
   h->d_bins = nullptr;
+  // now that the number of atoms is known, the block for it (48^3 order 4 at 0.173 atoms per grid point: 3 x 3
+  // rows 52 us; 4 x 4, the better at 0.1, 55)
+  s.set_fill(natom);
+  s.pick_block(sm_count(h->device));
   s.bin_cap = s.roomy_cap(cap);
   if (cudaMalloc(&h->d_bins, s.bin_ints(cap, s.bin_cap) * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
@@ -240,12 +250,6 @@ void set_config(pme_recip* h, const pme_tune_config& c) {
   h->st.tx_y = c.y_lines;
   h->st.tx_z = c.z_columns;
   h->grid_cap = c.grid_ctas;
-}
-
-int sm_count(int dev) {
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 1;
-  return sms;
 }
 
 // base * scale lines per pass tile, at most limit, shrunk (not below base) until the tile's

@@ -178,6 +178,7 @@ struct SystemState {
   int bry = 4, brz = 4, nby = 1, nbz = 1;
   int ctas = 0;              // CTAs per SM that the row blocks were chosen for: 2 the latency build, 3 the
                              // throughput build (0: shared launches, whose tile counts decide)
+  double fill = 0.1;         // atoms per grid point that the block costs assume
   int bin_cap = 0, atom_cap = 0;
   int* bins = nullptr;       // counts, bin records, bookkeeping, overflow records, atom order
   unsigned long long* accum = nullptr;
@@ -245,6 +246,10 @@ struct SystemState {
     nbz = (nz + brz - 1) / brz;
   }
 
+  // Liquid where the atoms are: natom over the whole grid, from 0.1 (water at 1 A; a box partly empty has
+  // as much in its filled part) to 0.2.
+  void set_fill(int natom) { fill = std::max(0.1, std::min(0.2, natom / (double)G())); }
+
   // The build for the block in place (after a change of the order).
   void pick_build(int sms) {
     const double three = block_cost(bry, brz, 3, sms);
@@ -267,7 +272,7 @@ struct SystemState {
     d.brz = bz;
     const size_t smem = c * (fused_smem_bytes(d) + 2064);   // the kernels' static part, what each CTA reserves
     if (smem > 228 * 1024) return 0.0;
-    const double tiles = (double)((ny + by - 1) / by) * ((nz + bz - 1) / bz), per_row = 0.1 * nx;
+    const double tiles = (double)((ny + by - 1) / by) * ((nz + bz - 1) / bz), per_row = fill * nx;
     const double cand = by * ((order - 2 + by) / by + 1) * bz * ((order - 2 + bz) / bz + 1);   // rows of the bins
     const double tile = 6.0 + per_row * (18.5e-3 * cand + 0.56e-3 * order * order * order * by * bz);
     const double two = order == 4 ? 0.78 : (order == 6 ? 0.76 : 0.70);

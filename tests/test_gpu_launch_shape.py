@@ -101,3 +101,27 @@ def test_changed_order_gives_a_new_handles_bits(cuda, nfft, first, order, evalua
         got = _eval(cuda, p, s, x)
         assert np.array_equal(got[0], want[0]) and got[1] == want[1] and np.array_equal(got[2], want[2])
     p.close()
+
+
+def test_row_block_follows_the_number_of_atoms(cuda):
+    """48^3 order 4: blocks of 4 x 4 rows (144 tiles) at 0.1 atoms per grid point, 3 x 3 (256) at 0.2; a
+    handle that grows from the one to the other takes the new block and keeps its results."""
+    from gpu_recip_b200 import CudaPMERecip
+    from gpu_recip_b200.pme import TRACE_STEP_STAMPS
+    sms = cuda.cuda.get_device_properties(0).multi_processor_count
+    if sms != 148:
+        pytest.skip("the tile counts are for 148 SMs")
+    p = CudaPMERecip(48, 48, 48, 4)
+    for waters, tiles in ((3700, 144), (7400, 256), (3700, 256)):
+        box = (48.0,) * 3
+        s = S.PmeSystem("atoms", S.water_box(waters, box, 6), box, (48, 48, 48), 4, 0.33)
+        x = cuda.from_numpy(s.xyzq).cuda()
+        buf = cuda.zeros(1024 * 14 + TRACE_STEP_STAMPS, dtype=cuda.int64, device="cuda")
+        p.set_trace(buf, 1024)
+        got = _eval(cuda, p, s, x)
+        p.set_trace(None)
+        # a CTA per tile (and one for the record)
+        assert int((buf[:1024 * 14].view(1024, 7, 2)[:, 1, 0] > 0).sum()) in (tiles, tiles + 1)
+        want = _eval(cuda, CudaPMERecip(48, 48, 48, 4), s, x, staged=True)
+        assert np.array_equal(got[0], want[0]) and got[1] == want[1] and np.array_equal(got[2], want[2])
+    p.close()
