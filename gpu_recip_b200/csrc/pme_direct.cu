@@ -35,11 +35,7 @@
 namespace pme {
 namespace direct {
 
-constexpr int kWarps = 4;             // warps per CTA of the pair kernel
-constexpr int kPairCtas = 5;          // its CTAs per SM
-constexpr int kQueue = 72;            // queued candidates per i atom (at most 32 more at a time)
 constexpr int kTasksPerWarp = 5;      // pair tasks per resident warp to aim at (24,000 atoms: 5 per warp 275 us a step, 3 279, 1 308)
-constexpr int kSquareTypes = 64;      // vdW types up to which every CTA holds the full square table
 constexpr int kMaxTypes = 200;        // vdW types
 constexpr float kEnergyScale = 4294967296.0f;     // 2^32
 constexpr float kForceScaleF = 1099511627776.0f;  // 2^40
@@ -319,6 +315,7 @@ __global__ void __launch_bounds__(kWarps * 32, kPairCtas) k_direct_pairs(
   __shared__ int2 sh_queue[kWarps][kCluster][kQueue + 1];   // j and its image (2 bits per axis)
   __shared__ ulonglong2 sh_xy[kWarps][kCluster / 2];        // the cluster's coordinates, atoms in pairs
   __shared__ unsigned long long sh_z[kWarps][kCluster / 2];
+  static_assert(sizeof(sh_queue) + sizeof(sh_xy) + sizeof(sh_z) == kPairShared, "what square_types counts");
   if (p.square)
     for (int k = threadIdx.x; k < p.ntype * p.ntype; k += blockDim.x) sh_vdw[k] = vdw_c6c12(vdwp, k / p.ntype, k % p.ntype);
   __syncthreads();
@@ -659,6 +656,7 @@ using namespace pme::direct;
 
 struct pme_direct {
   int device = 0;
+  int sm_shared = 0;         // the device's shared memory per SM, bytes
   cudaStream_t stream = nullptr;
   bool configured = false;
   double box[3] = {0, 0, 0};
@@ -732,7 +730,6 @@ Params make_params(const pme_direct* h) {
   p.vdw = h->vdw_model;
   p.elec = h->elec_model;
   p.ntype = h->ntype;
-  p.square = h->ntype <= kSquareTypes ? 1 : 0;
   const double big = 1024.0 / h->roff;
   long long big_bits;
   std::memcpy(&big_bits, &big, sizeof(big));
@@ -863,6 +860,7 @@ int pme_direct_create(void* stream, pme_direct** out) {
   cudaError_t e = cudaGetDevice(&h->device);
   h->stream = (cudaStream_t)stream;
   if (e == cudaSuccess) e = configure_pair_kernels(h->device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->sm_shared, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device);
   if (e == cudaSuccess && cudaMalloc(&h->d_acc, kAccN * sizeof(long long)) != cudaSuccess) e = cudaErrorMemoryAllocation;
   if (e == cudaSuccess) e = cudaMemset(h->d_acc, 0, kAccN * sizeof(long long));
   if (e != cudaSuccess) {
@@ -1068,11 +1066,12 @@ int pme_direct_calc_force(pme_direct* h, const void* xyzq, int ncoord, int calc_
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
   const bool ev = calc_energy || calc_virial;
+  const size_t table = (size_t)p.tab_n * (ev ? 2 : 1) * kTabTerms * sizeof(double);
+  p.square = square_types(p.ntype, table, h->sm_shared) ? 1 : 0;
   const bool std_terms = h->vdw_model != PME_VDW_NONE && p.square && p.tab_n > 0;
   auto kern = std_terms ? (ev ? k_direct_pairs<true, true> : k_direct_pairs<false, true>)
                         : (ev ? k_direct_pairs<true, false> : k_direct_pairs<false, false>);
-  const size_t smem = (size_t)p.tab_n * (ev ? 2 : 1) * kTabTerms * sizeof(double) +
-                      (size_t)(p.square ? p.ntype * p.ntype : 0) * sizeof(float2);
+  const size_t smem = table + (size_t)(p.square ? p.ntype * p.ntype : 0) * sizeof(float2);
   // one wave of resident CTAs; their warps draw the tasks from a counter.  Few clusters: more tasks
   // each, so that the last ones to finish are short
   int occ = 1;

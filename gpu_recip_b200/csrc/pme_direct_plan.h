@@ -58,6 +58,20 @@ inline Columns room_columns(const double* box, double roff, int natom) {
   return plan_columns(b, roff, (int)std::min(2147483647.0, std::ceil(f * f * f * natom)));
 }
 
+constexpr int kWarps = 4;             // warps per CTA of the pair kernel
+constexpr int kPairCtas = 5;          // its CTAs per SM
+constexpr int kQueue = 72;            // queued candidates per i atom (at most 32 more at a time)
+constexpr size_t kPairShared = kWarps * (kCluster * (kQueue + 1) * 8 + kCluster * 12);   // static, bytes
+
+// Whether every CTA holds the vdW parameters as a square of types in shared memory, beside table_bytes of
+// the Ewald table: while that leaves kPairCtas on an SM of sm_shared bytes.  The packed triangle is else
+// read through L1.  192,000 atoms at 9 A, us, square and packed: forces only 2 types 748 and 843, 40 (5
+// CTAs) 764 and 857, 48 (4) 868 and 863, 64 (3) 1,050 and 868; with energies 32 (5) 1,036 and 1,091, 40
+// (4) 1,128 and 1,091, 64 (3) 1,336 and 1,098.
+inline bool square_types(int ntype, size_t table_bytes, size_t sm_shared) {
+  return kPairCtas * (kPairShared + table_bytes + 8 * (size_t)ntype * ntype + 1024) <= sm_shared;
+}
+
 // Ewald table: polynomials on the intervals of s = r^2 that share their leading float bits, kTabOctave
 // per factor of two from s = 2 on, so that the interval is read off the bits.
 constexpr int kTabOctave = 32, kTabTerms = 6, kTabMax = 16 * kTabOctave;

@@ -48,9 +48,21 @@ static int ewald() {
   return 0;
 }
 
+// Ewald table bytes and shared memory per SM per line of stdin -> types up to which the square is held
+static int types() {
+  long long bytes, shared;
+  while (std::scanf("%lld %lld", &bytes, &shared) == 2) {
+    int n = 0;
+    while (square_types(n + 1, (size_t)bytes, (size_t)shared)) n++;
+    std::printf("%d\n", n);
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   if (argc == 2 && !std::strcmp(argv[1], "columns")) return columns();
   if (argc == 2 && !std::strcmp(argv[1], "sums")) return sums();
   if (argc == 2 && !std::strcmp(argv[1], "ewald")) return ewald();
+  if (argc == 2 && !std::strcmp(argv[1], "types")) return types();
   return 1;
 }

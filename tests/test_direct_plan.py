@@ -46,6 +46,15 @@ def test_columns_of_usual_systems(plan):
     assert [[int(v) for v in row[:4]] for row in out] == [[62, 13, 13, 2], [124, 27, 27, 2], [18, 3, 3, 2]]
 
 
+def test_square_of_types_keeps_the_ctas(plan):
+    """228 KB per SM, cutoffs of 9 and 12 A, forces only and with energies: the square of types takes what
+    five CTAs leave, and no more."""
+    tables = [171 * 48, 171 * 96, 199 * 48, 199 * 96]
+    most = [int(row[0]) for row in plan("types", [(t, 228 * 1024) for t in tables])]
+    assert most == [int(((228 * 1024) // 5 - 1024 - 19072 - t) // 8) ** 0.5 // 1 for t in tables]
+    assert most[0] > 40 and most[0] < 48 and most[1] > 32 and most[1] < 40
+
+
 @pytest.mark.parametrize("roff", [9.0, 12.0, 20.0])
 @pytest.mark.parametrize("kappa", [0.0, 0.25, 0.32, 0.45, 1.0])
 def test_ewald_table_errors(plan, kappa, roff):

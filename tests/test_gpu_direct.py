@@ -278,6 +278,31 @@ def test_direct_cluster_edges_match_oracle(cuda, oracle, box, n, roff, ntype, ka
     dr.close()
 
 
+@pytest.mark.parametrize("ntype", [30, 37, 38, 45, 46, 47, 48, 64, 65, 200])
+def test_types_that_no_atom_has_change_nothing(cuda, ntype):
+    """The same parameters in a table of 3 types (held as a square in shared memory) and in a larger one, on
+    both sides of where the square gives way to the packed triangle: the same forces, energies and virial."""
+    from gpu_recip_b200.direct import CudaPMEDirectForce
+    d = _lattice()
+    n = d["xyzq"].shape[0]
+    x = cuda.from_numpy(np.ascontiguousarray(d["xyzq"], dtype=np.float32)).cuda()
+    vp = np.zeros(ntype * (ntype + 1), np.float32)
+    vp[:12] = np.random.default_rng(4).random(12) * np.tile([1.0e2, 1.0e5], 6)
+    out = []
+    for m in (3, ntype):
+        dr = CudaPMEDirectForce()
+        dr.setup(24.0, 24.0, 24.0, 0.35, 9.0, 7.5, 1.0)
+        dr.set_vdwparam(vp[:m * (m + 1)])
+        dr.set_vdwtype(np.arange(n, dtype=np.int32) % 3)
+        f, e, v = _run(cuda, dr, x, n, n)
+        g = cuda.zeros(3 * n, dtype=cuda.int64, device="cuda")
+        dr.calc_force(x, n, False, False, n, g)
+        assert np.array_equal(f, g.view(3, n).T.cpu().numpy())
+        out.append((f, e, v))
+        dr.close()
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1] and np.array_equal(out[0][2], out[1][2])
+
+
 @pytest.mark.parametrize("box", [(40.0, 40.0, 40.0), (62.0, 70.0, 55.0)])
 def test_breathing_box_needs_no_new_work_space(cuda, box):
     """Edges up to 4% longer than at the first call: calc_force allocates nothing (an allocation ends a
