@@ -29,7 +29,7 @@
 
 #include "../../include/pme_direct.h"
 #include "pme_direct_plan.h"
-#include "pme_direct_sum.h"
+#include "pme_direct_math.h"
 #include "pme_state.h"
 
 namespace pme {
@@ -94,15 +94,6 @@ __device__ __forceinline__ float pair_terms(float r2, float qq, float c6, float 
 // The same terms in FP64 from the FP32 pair geometry, for the main pair list: the atoms' net
 // forces are small differences of large pair forces (close contacts of ~1e3 kcal/mol/A), where
 // the few-ulp error of an FP32 evaluation shows.
-
-// 1 / x by one third-order Newton (Halley-type) step y (1 + e + e^2), e = 1 - x y, from the
-// hardware's approximation (relative error below 2^-19, so below 2^-52 after the step).
-__device__ __forceinline__ double reciprocal(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = __fma_rn(-x, y, 1.0);
-  return __fma_rn(y, __fma_rn(e, e, e), y);
-}
 
 static_assert(kTabTerms == 6, "quintics");
 __device__ __forceinline__ double quintic(const double2* c, double t) {

@@ -1,5 +1,5 @@
-// pme_direct_sum.h -- exact sums of the pair kernel's force terms, each rounded once to 2^-40.  Plain C++
-// beside CUDA, so that the arithmetic can be checked without a GPU.
+// pme_direct_math.h -- arithmetic of the pair kernel: exact sums of its force terms, each rounded once to
+// 2^-40 (plain C++ beside CUDA, so that they can be checked without a GPU), and its reciprocal.
 #pragma once
 
 #include <cstring>
@@ -36,6 +36,23 @@ struct RoundedSum {
     return bits - (unsigned long long)rounded_terms * bits_of(kRoundMagic);
   }
 };
+
+#ifdef __CUDACC__
+// The hardware's approximation of 1 / x, |1 - x y| < 2^-19 (its 20 leading mantissa bits; measured in
+// tests/test_gpu_direct_math.py).
+__device__ __forceinline__ double reciprocal_guess(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+
+// 1 / x by one third-order Newton (Halley-type) step y (1 + e + e^2), e = 1 - x y, from the guess: e^3 <
+// 2^-57 is left, so the result is within an ulp of 1 / x.
+__device__ __forceinline__ double reciprocal(double x) {
+  const double y = reciprocal_guess(x), e = __fma_rn(-x, y, 1.0);
+  return __fma_rn(y, __fma_rn(e, e, e), y);
+}
+#endif
 
 }  // namespace direct
 }  // namespace pme

@@ -4,7 +4,7 @@
 #include <cstring>
 
 #include "pme_direct_plan.h"
-#include "pme_direct_sum.h"
+#include "pme_direct_math.h"
 
 using namespace pme::direct;
 

@@ -1,5 +1,5 @@
 """The direct-space engine's host-side choices (csrc/pme_direct_plan.h) and exact sums
-(csrc/pme_direct_sum.h), compiled with the undefined behaviour sanitizer and checked without a GPU."""
+(csrc/pme_direct_math.h), compiled with the undefined behaviour sanitizer and checked without a GPU."""
 import itertools
 import os
 import subprocess
