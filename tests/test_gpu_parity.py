@@ -39,7 +39,7 @@ def _sys(name):
     if name == "long_z":      # nz > 256: the fused path runs separate y / z passes, not plane tiles
         box = (15.0, 16.0, 300.0)
         return S.PmeSystem("lz", S.water_box(1500, box, 34), box, (16, 18, 320), 4, 0.35)
-    if name == "bigq":        # two charges of +-700: the fused tile leaves its 2-sum accumulation form
+    if name == "bigq":        # two charges of +-700: at the bound of the fused tile's 2-sum accumulation form
         s = _sys("odd_grid")
         x = s.xyzq.copy()
         x[0, 3], x[1, 3] = 700.0, -700.0
@@ -152,9 +152,10 @@ def test_reference_fixture(cuda, ref_fixture, order):
                                            ("dense_p8", 0)])
 def test_staged_calls_equal_fused_eval(cuda, name, schedule):
     """Staged reference-style calls and the fused kernel (either y/z schedule) agree bit for bit.
-    The fused tile accumulates its charge rows in one of three exact forms, chosen from the tile's
-    candidate count and the largest |q|; water boxes take the 2-sum form, bigq the 3-sum form and
-    dense_p8 the carry form, and all must give the staged path's int64 grid."""
+    The fused tile accumulates its charge rows in one of two exact forms, chosen from the tile's
+    candidate count and the largest |q|; water boxes take the 2-sum form, dense_p8 (more than 65,536
+    candidates per tile) the carry form, bigq's charges lie at the bound between the two, and all must
+    give the staged path's int64 grid."""
     s = _sys(name)
     a = _run(cuda, s, staged=True)
     pme = _pme(cuda, s)
