@@ -54,8 +54,8 @@ struct pme_recip {
   int plane_mode = 0;   // 0 automatic, 1 whole-plane tiles where they fit, 2 separate passes
   int grid_cap = 0;     // CTAs of the persistent launch (0: as many as are resident)
   int x_gather = PME_XGATHER_AUTO;   // PME_XGATHER_*
-  bool accum_zero = true;
-  bool no_cluster = false;   // the cluster launch of the plane phase could not be shaped here    // the int64 charge grid is known to be all zero (staged spread skips its clear)
+  bool accum_zero = true;    // the int64 charge grid is known to be all zero (staged spread skips its clear)
+  bool no_cluster = false;   // the cluster launch of the plane phase could not be shaped here
   float* d_force = nullptr;      // pme_eval_host: device forces before the copy to the host
   size_t force_bytes = 0;
 };
@@ -160,8 +160,7 @@ int launch_fused_single(pme_recip* h, const SysDesc& d_in) {
   if (h->trace) d.steps = h->trace + (size_t)h->trace_ctas * kPhases * 2;
   // whole-plane tiles only pay when there are enough planes to occupy the GPU; otherwise the
   // separate y and z passes spread the same work over many more CTAs
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+  const int sms = sm_count(h->device);
   if (h->plane_mode == 0) d.plane = (d.plane && d.g.hx >= sms) ? 1 : 0;
   else d.plane = (d.plane && h->plane_mode == 1) ? 1 : 0;
   // fewer full bin tiles than SMs: half-size tiles, so that no SM bins more than kThreads atoms

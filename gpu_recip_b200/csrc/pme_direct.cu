@@ -654,7 +654,7 @@ struct pme_direct {
   double kappa = 0, roff = 0, ron = 0, e14fac = 1.0;
   int vdw_model = PME_VDW_VSH, elec_model = PME_ELEC_EWALD;
   // tables
-  int ntype = 0, ntype14 = 0, npair = 0, npair14 = 0;
+  int ntype = 0, ntype14 = 0;
   float2* d_vdw = nullptr;
   float2* d_vdw14 = nullptr;
   int n_types = 0;           // atoms of the vdW type table, and its largest type
@@ -834,8 +834,7 @@ int upload_vdw(pme_direct* h, int nvdwparam, const float* hp, bool in14) {
   DeviceGuard dg(h->device);
   cudaError_t e = upload(in14 ? &h->d_vdw14 : &h->d_vdw, t.data(), t.size(), h->stream);
   if (e != cudaSuccess) return cuda_fail(e, "vdwparam: upload");
-  if (in14) { h->npair14 = npair; h->ntype14 = ntype; }
-  else { h->npair = npair; h->ntype = ntype; }
+  (in14 ? h->ntype14 : h->ntype) = ntype;
   return PME_OK;
 }
 

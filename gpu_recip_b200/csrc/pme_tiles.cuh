@@ -111,7 +111,6 @@ __host__ __device__ inline int tiles_bin(const SysDesc& d) { return (d.natom + b
 __host__ __device__ inline int tiles_blocks(const SysDesc& d) { return d.nby * d.nbz; }
 // Lanes per atom of the gather (staged and fused): one per stencil column along x, a power of two.
 __host__ __device__ constexpr int gather_lanes(int order) { return order <= 4 ? 4 : 8; }
-constexpr int kGatherAtoms = kThreads / 8;   // staged gather tile: atoms of the smallest pass
 __host__ __device__ inline int tiles_gather(const SysDesc& d) {
   const int app = kThreads / gather_lanes(d.order);
   return (d.natom + app - 1) / app;
@@ -1423,8 +1422,8 @@ __device__ __forceinline__ void gather_tile(const SysDesc& d, int tile) {
 }
 
 // Fused path: gather the atoms of one row-block bin (plus the overflow atoms whose origin lies in
-// the block), kGatherAtoms at a time, so that the tile's stencil rows (about
-// (4+P-1)^2 grid rows) stay in L1.  Atoms come from the bin's records (origin, fractional offsets
+// the block), as many at a time as have their lanes, so that the tile's stencil rows (at most
+// (bry+P-1)(brz+P-1) grid rows) stay in L1.  Atoms come from the bin's records (origin, fractional offsets
 // and charge, so no coordinate reload), the next pass's records loading while the current ones are
 // gathered.  The tile also writes its atoms into the system's bin-sorted atom order at the bin's
 // offset; the next evaluation's binning walks the atoms in that order, so that the atoms of a warp
