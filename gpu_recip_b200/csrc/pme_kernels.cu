@@ -57,10 +57,15 @@ __global__ void __launch_bounds__(kThreads) k_spread(const __grid_constant__ Sys
   spread_dispatch(d, blockIdx.x, smem);
 }
 
-__global__ void __launch_bounds__(kThreads) k_gather(const __grid_constant__ SysDesc p) {
+// A kernel per order, with registers for 4 (order 4) or 3 CTAs per SM: one kernel for all orders has the 98
+// registers of order 8 and 2 CTAs, too few to cover the loads of atoms in any order.  us, one for all and
+// as here: 1,008,000 atoms on 216^3 order 4 139 and 96 (5 CTAs: 92, but 3,000 atoms 5.0 for 4.4), order 6 329
+// and 278, order 8 727 and 400; 24,000 atoms on 64^3 order 4 8.5 and 6.5, order 8 23.9 and 15.7.
+template <int P>
+__global__ void __launch_bounds__(kThreads, P <= 4 ? 4 : 3) k_gather(const __grid_constant__ SysDesc p) {
   __shared__ SysDesc d;
   load_desc(d, p);
-  gather_dispatch(d, blockIdx.x);
+  gather_tile_any<P>(d, blockIdx.x);
 }
 
 // ------------------------------- fused persistent kernel --------------------------------------
@@ -445,7 +450,9 @@ cudaError_t staged_c2r(const SysDesc& d, const StagedCtx& c, cudaStream_t s) {
 cudaError_t staged_gather(const SysDesc& d, cudaStream_t s) {
   const int blocks = tiles_gather(d);
   if (blocks <= 0) return cudaSuccess;
-  k_gather<<<blocks, kThreads, 0, s>>>(d);
+  if (d.order == 4) k_gather<4><<<blocks, kThreads, 0, s>>>(d);
+  else if (d.order == 6) k_gather<6><<<blocks, kThreads, 0, s>>>(d);
+  else k_gather<8><<<blocks, kThreads, 0, s>>>(d);
   return cudaGetLastError();
 }
 

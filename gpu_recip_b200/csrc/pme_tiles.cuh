@@ -1584,14 +1584,6 @@ __device__ __forceinline__ void gather_tile_any(const SysDesc& d, int tile) {
   }
 }
 
-__device__ __forceinline__ void gather_dispatch(const SysDesc& d, int tile) {
-  switch (d.order) {
-    case 4: gather_tile_any<4>(d, tile); break;
-    case 6: gather_tile_any<6>(d, tile); break;
-    default: gather_tile_any<8>(d, tile); break;
-  }
-}
-
 template <int P, bool GX>
 __device__ __forceinline__ void gather_bin_any(const SysDesc& d, int tile, int parity, char* smem) {
   switch (d.force_kind) {
