@@ -234,7 +234,7 @@ struct SystemState {
         if (need > kTileSmemBudget || (sms == 0 && best > 0.0)) continue;
         for (int c = 2; c <= (sms > 0 ? 3 : 2); c++) {
           const double cost = sms > 0 ? block_cost(by, bz, c, sms) : 1.0;
-          if (cost > 0.0 && (best == 0.0 || cost < best)) {
+          if (cost > 0.0 && (best == 0.0 || cost < best)) {   // (the latency build always has a cost)
             best = cost;
             bry = by;
             brz = bz;
@@ -256,8 +256,8 @@ struct SystemState {
     ctas = three > 0.0 && three < block_cost(bry, brz, 2, sms) ? 3 : 2;
   }
 
-  // Estimated cost of an evaluation's row-block tiles, by x bz rows each and c CTAs per SM; 0 where c do not
-  // fit.  A tile costs 6 + 18.5e-3 per candidate record (of every bin that its window touches) + 0.56e-3
+  // Estimated cost of an evaluation's row-block tiles, by x bz rows each, in the build for c CTAs per SM (2: the
+  // latency build, which takes one where two do not fit); 0 where three do not fit.  A tile costs 6 + 18.5e-3 per candidate record (of every bin that its window touches) + 0.56e-3
   // per contribution with 3 CTAs on its SM, less with fewer beside it: 0.76 to 0.78 of that with 2 (0.70 at
   // order 8), 0.55 alone; 6% more where the SM's shared memory grows beyond 196 KB, to its largest size,
   // and leaves the gather less L1.  Fitted to whole evaluations of 267 systems (18^3 to 216^3, uneven ones
@@ -270,14 +270,15 @@ struct SystemState {
     d.plane = 0;
     d.bry = by;
     d.brz = bz;
-    const size_t smem = c * (fused_smem_bytes(d) + 2064);   // the kernels' static part, what each CTA reserves
-    if (smem > 228 * 1024) return 0.0;
+    const size_t smem = fused_smem_bytes(d) + 2064;   // the kernels' static part, what each CTA reserves
+    const int fit = std::max(1, std::min(c, (int)(228 * 1024 / smem)));
+    if (c == 3 && fit < 3) return 0.0;
     const double tiles = (double)((ny + by - 1) / by) * ((nz + bz - 1) / bz), per_row = fill * nx;
     const double cand = by * ((order - 2 + by) / by + 1) * bz * ((order - 2 + bz) / bz + 1);   // rows of the bins
     const double tile = 6.0 + per_row * (18.5e-3 * cand + 0.56e-3 * order * order * order * by * bz);
     const double two = order == 4 ? 0.78 : (order == 6 ? 0.76 : 0.70);
-    const double share = c == 3 ? 1.0 : (tiles <= sms ? 0.55 : two);
-    return std::ceil(tiles / (c * sms)) * tile * share * (smem > 196 * 1024 ? 1.06 : 1.0) + (c == 3 ? 1.0 : 0.0);
+    const double share = c == 3 ? 1.0 : (fit == 1 || tiles <= sms ? 0.55 : two);
+    return std::ceil(tiles / (fit * sms)) * tile * share * (fit * smem > 196 * 1024 ? 1.06 : 1.0) + (c == 3 ? 1.0 : 0.0);
   }
 
   int nbins() const { return nby * nbz; }

@@ -125,3 +125,26 @@ def test_row_block_follows_the_number_of_atoms(cuda):
         want = _eval(cuda, CudaPMERecip(48, 48, 48, 4), s, x, staged=True)
         assert np.array_equal(got[0], want[0]) and got[1] == want[1] and np.array_equal(got[2], want[2])
     p.close()
+
+
+@pytest.mark.parametrize("nfft,order", [((16, 512, 512), 4), ((24, 400, 360), 8)])
+def test_grids_whose_tiles_leave_one_cta_per_sm(cuda, nfft, order):
+    """The z tiles of long y and z axes take more than half an SM's shared memory: the row block is still
+    one of many rows (an evaluation with blocks of one row took 20 to 40 times the staged calls), and the
+    bits are theirs."""
+    from gpu_recip_b200 import CudaPMERecip
+    s = _system(nfft, order)
+    x = cuda.from_numpy(s.xyzq).cuda()
+    p = CudaPMERecip(*nfft, order)
+    ms, out = [], []
+    for staged in (False, True):
+        for k in range(4):
+            a, b = cuda.cuda.Event(enable_timing=True), cuda.cuda.Event(enable_timing=True)
+            a.record()
+            got = _eval(cuda, p, s, x, staged)
+            b.record()
+            b.synchronize()
+        ms.append(a.elapsed_time(b))
+        out.append(got)
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1] == out[1][1] and np.array_equal(out[0][2], out[1][2])
+    assert ms[0] < 4.0 * ms[1], ms
