@@ -64,12 +64,14 @@ constexpr int kQueue = 72;            // queued candidates per i atom (at most 3
 constexpr size_t kPairShared = kWarps * (kCluster * (kQueue + 1) * 8 + kCluster * 12);   // static, bytes
 
 // Whether every CTA holds the vdW parameters as a square of types in shared memory, beside table_bytes of
-// the Ewald table: while that leaves kPairCtas on an SM of sm_shared bytes.  The packed triangle is else
-// read through L1.  192,000 atoms at 9 A, us, square and packed: forces only 2 types 748 and 843, 40 (5
-// CTAs) 764 and 857, 48 (4) 868 and 863, 64 (3) 1,050 and 868; with energies 32 (5) 1,036 and 1,091, 40
-// (4) 1,128 and 1,091, 64 (3) 1,336 and 1,098.
+// the Ewald table: while that costs none of the CTAs on an SM of sm_shared bytes (kPairCtas; fewer with
+// energies beyond a cutoff of 29 A).  The packed triangle is else read through L1.  192,000 atoms at 9 A,
+// us, square and packed: forces only 2 types 748 and 843, 40 (5 CTAs) 764 and 857, 48 (4) 868 and 863, 64
+// (3) 1,050 and 868; with energies 32 (5) 1,036 and 1,091, 40 (4) 1,128 and 1,091, 64 (3) 1,336 and 1,098;
+// 24,000 atoms at 32 A with energies, 2 types (4) 3,877 and 4,361.
 inline bool square_types(int ntype, size_t table_bytes, size_t sm_shared) {
-  return kPairCtas * (kPairShared + table_bytes + 8 * (size_t)ntype * ntype + 1024) <= sm_shared;
+  const size_t without = kPairShared + table_bytes + 1024, with = without + 8 * (size_t)ntype * ntype;
+  return with <= sm_shared && sm_shared / with >= std::min((size_t)kPairCtas, sm_shared / without);
 }
 
 // Ewald table: polynomials on the intervals of s = r^2 that share their leading float bits, kTabOctave

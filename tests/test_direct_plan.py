@@ -53,6 +53,9 @@ def test_square_of_types_keeps_the_ctas(plan):
     most = [int(row[0]) for row in plan("types", [(t, 228 * 1024) for t in tables])]
     assert most == [int(((228 * 1024) // 5 - 1024 - 19072 - t) // 8) ** 0.5 // 1 for t in tables]
     assert most[0] > 40 and most[0] < 48 and most[1] > 32 and most[1] < 40
+    # a long cutoff (60 A, with energies: 345 intervals) leaves fewer CTAs anyway: a few types cost none of them
+    assert 5 * (19072 + 1024 + 345 * 96) > 228 * 1024
+    assert int(plan("types", [(345 * 96, 228 * 1024)])[0][0]) >= 25
 
 
 @pytest.mark.parametrize("roff", [9.0, 12.0, 20.0])
