@@ -167,6 +167,11 @@ int launch_fused_single(pme_recip* h, const SysDesc& d_in) {
   // where the hardware doubles CTAs up (measured on 24,000 atoms: 0.9 us faster; 64-atom tiles
   // were 2 us slower)
   d.bin_atoms = (d.natom + kThreads - 1) / kThreads < sms ? kThreads / 2 : kThreads;
+  // the build that the row block was chosen for; the latency build where the caller asks for cluster planes,
+  // which no other has
+  const bool cluster_fits = !h->no_cluster && !d.g.tric && d.g.ny % kClusterPlane == 0 && d.g.nz % kClusterPlane == 0 &&
+                            cplane_smem_bytes(d.g.ny, d.g.nz, kClusterPlane) <= kTileSmemBudget;
+  const int ctas = h->plane_mode == PME_SCHED_CLUSTER && cluster_fits ? 2 : h->st.ctas;
   // inverse x pass inside the gather tiles where its rows fit in the shared memory the other
   // phases already take (so that the launch keeps its CTAs per SM)
   // (latency build only: the throughput build keeps the separate phase and is compiled without the
@@ -174,12 +179,12 @@ int launch_fused_single(pme_recip* h, const SysDesc& d_in) {
   // transformed again by every tile, 2 to 4 times the phase's work, which a second wave does not hide
   // (order 4, fused and separate: 40^3, 196 tiles, 45.6 and 46.3 us; 64^3, 256, 48.3 and 48.2; 72^3,
   // 324, 85.4 and 81.3; 576 tiles 94.4 and 85.8)
-  d.gx = h->x_gather == PME_XGATHER_AUTO && h->st.ctas <= 2 && tiles_blocks(d) <= 2 * sms &&
+  d.gx = h->x_gather == PME_XGATHER_AUTO && ctas <= 2 && tiles_blocks(d) <= 2 * sms &&
                  gx_smem_bytes(d.g.nx, d.bry, d.brz, d.order) <= fused_smem_bytes(d) ? 1 : 0;
   fused_tile_counts(d, a.total);
   size_t smem = fused_smem_bytes(d);
   FusedShape shape;
-  cudaError_t e = fused_shape(a.total, smem, h->grid_cap, h->st.ctas, &shape);
+  cudaError_t e = fused_shape(a.total, smem, h->grid_cap, ctas, &shape);
   if (e != cudaSuccess) return cuda_fail(e, "fused: launch shape (does the kernel fit on an SM?)");
   // y, z, the solve and both inverses as kx planes split over 4-CTA clusters, where the plane
   // count alone would leave most SMs idle (latency build, orthorhombic, line counts divisible);
@@ -187,8 +192,7 @@ int launch_fused_single(pme_recip* h, const SysDesc& d_in) {
   // 43.5 against 41.5 us with one CTA per plane)
   const bool want_cluster = h->plane_mode == PME_SCHED_CLUSTER ||
                             (h->plane_mode == PME_SCHED_AUTO && !d.plane && d.g.hx >= 32);
-  if (want_cluster && !h->no_cluster && shape.variant == kFusedLatency && !d.g.tric && d.g.ny % kClusterPlane == 0 &&
-      d.g.nz % kClusterPlane == 0 && cplane_smem_bytes(d.g.ny, d.g.nz, kClusterPlane) <= kTileSmemBudget) {
+  if (want_cluster && cluster_fits && shape.variant == kFusedLatency) {
     SysDesc c = d;
     c.plane = 0;
     c.cplane = kClusterPlane;

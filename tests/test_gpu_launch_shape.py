@@ -64,6 +64,25 @@ def test_build_follows_the_row_blocks(cuda, nfft, order, three, fused_x):
     p.close()
 
 
+@pytest.mark.parametrize("schedule,z_passes", [(0, True), (3, False)])
+def test_cluster_planes_asked_for_are_run(cuda, schedule, z_passes):
+    """72^3 order 4 runs the throughput build by itself, with y and z passes; the cluster planes, which only
+    the latency build has, where the caller asks for them."""
+    from gpu_recip_b200 import CudaPMERecip
+    from gpu_recip_b200.pme import TRACE_STEP_STAMPS
+    s = _system((72, 72, 72), 4)
+    x = cuda.from_numpy(s.xyzq).cuda()
+    p = CudaPMERecip(72, 72, 72, 4)
+    p.set_fft_schedule(schedule)
+    buf = cuda.zeros(1024 * 14 + TRACE_STEP_STAMPS, dtype=cuda.int64, device="cuda")
+    p.set_trace(buf, 1024)
+    got = _eval(cuda, p, s, x)
+    p.set_trace(None)
+    assert bool((buf[:1024 * 14].view(1024, 7, 2)[:, 3, 0] > 0).any()) == z_passes
+    want = _eval(cuda, CudaPMERecip(72, 72, 72, 4), s, x, staged=True)
+    assert np.array_equal(got[0], want[0]) and got[1] == want[1] and np.array_equal(got[2], want[2])
+
+
 def test_changed_order_takes_its_own_row_block(cuda):
     """Order 8 on 32^3 has blocks of 4 x 1 rows (256 tiles), order 4 of 3 x 3 (121): a handle whose order
     changes before its first evaluation is launched as one made with that order."""
